@@ -11,23 +11,36 @@
 // loop stops once more than targetSize points are accepted.
 //
 // Here one CTA runs one iteration and reproduces that sequence exactly. It
-// takes the candidates a block of 208 at a time (208 x 3 = 624 draws: one
-// MT19937 state block; word i >= 227 depends only on word i - 227, so 227
-// threads each compute a chain of up to three words, while warp 0 walks the
-// previous block), with three barriers per block:
-//   1. every thread of a candidate computes its position and its density in
-//      FP32, re-tested with the reference's sampler arithmetic (float voxel
-//      values, double weights, a float result per interpolation step) when
-//      the FP32 value is within its error bound of the cutoff;
-//   2. between two radius updates, every density-passing candidate is tested
-//      in parallel (a warp per candidate, lanes over the accepted points)
-//      against the points accepted before the segment;
-//   3. one lane walks the survivors in candidate order, testing each against
-//      the points accepted earlier in the same segment, and accepts.
+// takes the candidates a chunk at a time (3328 or 1664 of them), split where a
+// radius update falls inside one, so that the radius is one number in each
+// range:
+//   1. warps take groups of 64 candidates from a counter: position in FP32 index
+//      space, one cell record, density test. A candidate whose density or
+//      cell the FP32 error leaves undecided is tested again with an index
+//      position of two floats, and if need be with the reference's arithmetic
+//      (FP64 position, double weights, a float result per interpolation step).
+//      Those that pass are tested against two accepted points: the ones that
+//      last rejected candidates of the same hint cell (19 in 20 end here).
+//      Meanwhile eight warps first make the next chunk's MT19937 words;
+//   2. a warp per remaining candidate forms its position exactly as the
+//      reference rounds it (position_exact) and tests it against the accepted
+//      points in the cells of a kDartGrid^3 grid within the radius, a lane per
+//      cell. A radius change needs no rebuilding: the cells hold positions
+//      alone, and a hint is an accepted point wherever it is;
+//   3. warp 0 walks the survivors in candidate order, testing each against
+//      the points accepted in the same range, and accepts.
 // Distances are compared in FP32 and re-tested in FP64 (the reference's
 // arithmetic) when within 2^-18 of the squared radius, so the accepted set
 // is the reference's. The accepted points live in shared memory.
+//
+// What bounds it: latency, the steps of a range one after the other with a
+// barrier between (an iteration's ranges are a chain). Chunks of 208
+// candidates (one state block) with every listed candidate tested against all
+// accepted points by a warp and FP64 positions for every candidate took
+// 44.6 ms for 48 iterations of 1M candidates (256^3 cumulus); this form takes
+// 4.8 ms, and 500 iterations 16.4 ms instead of 76.
 #include <algorithm>
+#include <cmath>
 
 #include "lg_kernels.h"
 #include "lg_mt.h"
@@ -36,14 +49,15 @@ namespace lg {
 
 namespace {
 
-constexpr int kDartThreads = 512;  // >= 227 (the twist chains); 4 CTAs per SM
-constexpr int kDartBlock = 208;    // candidates per MT block (3 draws each)
-constexpr int kDartWarps = kDartThreads / 32;
+constexpr int kDartTwisters = 256;  // >= 227 threads that make the next words (the last eight warps)
+constexpr int kDartGrid = 16;  // cells per axis over the points' bbox
+constexpr int kDartHint = 20;  // hint cells per axis
+constexpr uint16_t kNoPoint = 0xFFFFu;
 
 // BoxSampler::sample restated as the reference evaluates it: float voxel
 // values, double weights, each interpolation rounded to float (z, then y,
 // then x). p is the index-space position.
-__device__ float sample_exact(const DevGrid& g, double px, double py, double pz) {
+__device__ __noinline__ float sample_exact(const DevGrid& g, double px, double py, double pz) {
     const double fx = floor(px), fy = floor(py), fz = floor(pz);
     const double u = px - fx, w = py - fy, t = pz - fz;
     float v[8];
@@ -68,249 +82,523 @@ __device__ float sample_exact(const DevGrid& g, double px, double py, double pz)
     return lerp(x0, x1, u);
 }
 
-// The density test without FP64 in the common case: an FP32 sample, and the
-// exact sample_exact when the FP32 value lies within its error bound of the
-// cutoff or the FP32 position lies within twice its error of a cell face
-// (where the exact position may sit in the neighbouring cell). Inside one
-// cell the trilinear sample moves by at most 3 * (max tap - min tap) per voxel
-// of position error index_err (FP32 rounding of wo, of 1 / h and of the
-// subtraction and product); the seven FP32 interpolations add under 2^-19 of
-// the largest tap. For an FP32 record (the polynomial k0 + ...) S = sum of
-// |k| over the non-constant terms stands in for the taps' spread: every
-// partial derivative is at most S and every tap lies within S of k0, so
-// |k0| + S bounds every tap; the coefficients' FP32 differences (54 * 2^-24
-// of the largest tap), their four evaluation steps and the exact sample's own
-// roundings stay under 4e-6 of |k0| + S, and the bound takes twice that.
-__device__ __forceinline__ bool density_passes(const DevGrid& g, const float p[3], const DartParams& prm) {
-    const float ix = (p[0] - prm.wo_f[0]) * prm.inv_h_f, iy = (p[1] - prm.wo_f[1]) * prm.inv_h_f,
-                iz = (p[2] - prm.wo_f[2]) * prm.inv_h_f;
+// The slow paths stay out of line: the kernel's steps are run in turn by every
+// warp, so its code should fit the instruction cache.
+__device__ __noinline__ float position_fp64(double bbmin, float x) {
+    return __double2float_rn(__dadd_rn((double)x, bbmin));
+}
+
+// The candidate's coordinate as the reference rounds it,
+// float(double(x) + bbmin) with x = float(u * size), for axis a. bbmin is
+// hi + lo to within 2^-48 of itself; x + hi = s + e exactly (two-sum), and
+// where s + (e + lo) rounds the same way after moving e + lo by more than
+// every rounding left out, that is the answer. Otherwise FP64 decides (its
+// additions and conversions run at 1/64 of the FP32 rate, which made them
+// most of the time when every candidate used them).
+__device__ __forceinline__ float position_exact(const DartParams& prm, int a, float x) {
+    const float hi = prm.bb_hi[a];
+    const float s = __fadd_rn(x, hi);
+    const float bb = __fsub_rn(s, x);
+    const float e = __fadd_rn(__fsub_rn(x, __fsub_rn(s, bb)), __fsub_rn(hi, bb));
+    const float t = __fadd_rn(e, prm.bb_lo[a]);
+    const float m = __fmaf_rn(fabsf(t), 2.384185791015625e-7f, prm.bb_err[a]);  // 2^-22
+    const float r0 = __fadd_rn(s, __fsub_rn(t, m)), r1 = __fadd_rn(s, __fadd_rn(t, m));
+    if (r0 == r1) return r0;
+    return position_fp64(prm.bbmin[a], x);
+}
+
+// Position offsets from bbmin of the candidate whose three words are at w.
+__device__ __forceinline__ void candidate_offsets(const DartParams& prm, const uint32_t* w, float x[3]) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) x[a] = __fmul_rn(mt_canonical_float(mt_temper(w[a])), prm.bbsize[a]);
+}
+
+// Its exact position.
+__device__ __forceinline__ void candidate_position(const DartParams& prm, const uint32_t* w, float p[3]) {
+    candidate_offsets(prm, w, p);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) p[a] = position_exact(prm, a, p[a]);
+}
+
+// The cell record and weights under a candidate in FP32: index = x / h +
+// (bbmin - wo) / h, off by at most prm.index_err voxels.
+struct DartCell {
+    float u, w, t;
+    uint32_t rec;
+};
+__device__ __forceinline__ DartCell candidate_cell(const DevGrid& g, const DartParams& prm, const float x[3]) {
+    const float ix = fmaf(x[0], prm.inv_h_f, prm.index0[0]), iy = fmaf(x[1], prm.inv_h_f, prm.index0[1]),
+                iz = fmaf(x[2], prm.inv_h_f, prm.index0[2]);
     const float fx = floorf(ix), fy = floorf(iy), fz = floorf(iz);
-    const float u = ix - fx, w = iy - fy, t = iz - fz;
-    float v[8];
-    const uint32_t rec = cell_record(g, (int)fx, (int)fy, (int)fz);
+    return {ix - fx, iy - fy, iz - fz, cell_record(g, (int)fx, (int)fy, (int)fz)};
+}
+
+__device__ __noinline__ float density_exact(const DevGrid& g, const DartParams& prm, float x, float y, float z) {
+    const double px = ((double)position_fp64(prm.bbmin[0], x) - prm.wo[0]) / prm.h;
+    const double py = ((double)position_fp64(prm.bbmin[1], y) - prm.wo[1]) / prm.h;
+    const double pz = ((double)position_fp64(prm.bbmin[2], z) - prm.wo[2]) / prm.h;
+    return sample_exact(g, px, py, pz);
+}
+
+// The density test in FP32: 0 fails, 1 passes, 2 undecided -- the value lies
+// within its error bound of the cutoff or the position within twice its error
+// of a cell face (where the exact position may sit in the neighbouring cell).
+// Inside one cell the trilinear sample moves by at most 3 * (max tap - min
+// tap) per voxel of position error index_err; the seven FP32 interpolations
+// add under 2^-19 of the largest tap. For an FP32 record (the polynomial k0 +
+// ...) S = sum of |k| over the non-constant terms stands in for the taps'
+// spread: every partial derivative is at most S and every tap lies within S of
+// k0, so |k0| + S bounds every tap; the coefficients' FP32 differences
+// (54 * 2^-24 of the largest tap), their four evaluation steps and the exact
+// sample's own roundings stay under 4e-6 of |k0| + S, and the bound takes twice
+// that.
+template <int DT>
+__device__ __forceinline__ int density_test(const DartCell& c, const float v[8], float index_err, float cutoff) {
     float val, spread, mag, rel = 2e-6f;
-    if (g.dtype == 0) {
+    if (DT == 0) {
         rel = 8e-6f;
-        ld_cell<0>(g.data, rec, v);
-        val = trilinear_coefs(v, u, w, t);
+        val = trilinear_coefs(v, c.u, c.w, c.t);
         float sum = 0.f;
 #pragma unroll
         for (int k = 1; k < 8; ++k) sum += fabsf(v[k]);
         spread = sum * (1.f + 1e-6f);
         mag = fabsf(v[0]) + spread;
     } else {
-        if (g.dtype == 1) ld_cell<1>(g.data, rec, v);
-        else ld_cell<2>(g.data, rec, v);
         float lo = v[0], hi = v[0];
 #pragma unroll
         for (int k = 1; k < 8; ++k) { lo = fminf(lo, v[k]); hi = fmaxf(hi, v[k]); }
         auto lerp = [](float a, float b, float wt) { return fmaf(b - a, wt, a); };
-        const float x0 = lerp(lerp(v[0], v[4], t), lerp(v[2], v[6], t), w);
-        const float x1 = lerp(lerp(v[1], v[5], t), lerp(v[3], v[7], t), w);
-        val = lerp(x0, x1, u);
+        const float x0 = lerp(lerp(v[0], v[4], c.t), lerp(v[2], v[6], c.t), c.w);
+        const float x1 = lerp(lerp(v[1], v[5], c.t), lerp(v[3], v[7], c.t), c.w);
+        val = lerp(x0, x1, c.u);
         spread = hi - lo;
         mag = fmaxf(fabsf(hi), fabsf(lo));
     }
-    const float e2 = 2.f * prm.index_err;
-    const bool near_face = u < e2 || u > 1.f - e2 || w < e2 || w > 1.f - e2 || t < e2 || t > 1.f - e2;
-    const float bound = 3.f * spread * prm.index_err + mag * rel + 1e-30f;
-    if (!near_face) {
-        if (val < prm.cutoff - bound) return false;
-        if (val > prm.cutoff + bound) return true;
+    const float e2 = 2.f * index_err;
+    if (fminf(fminf(c.u, c.w), c.t) < e2 || fmaxf(fmaxf(c.u, c.w), c.t) > 1.f - e2) return 2;
+    const float bound = 3.f * spread * index_err + mag * rel + 1e-30f;
+    return val < cutoff - bound ? 0 : val > cutoff + bound ? 1 : 2;
+}
+
+// The same with the index position (p - wo) / h of the exact p carried as a
+// sum of two floats, off by at most prm.index_err2 voxels: about one candidate
+// in 700 comes here for lying near a cell face, one in a million is left for
+// FP64, whose dependent steps at 1/64 of the FP32 rate made a whole range
+// wait (48 iterations of 1M candidates: 7.7 ms with FP64 alone, 5.6 ms so).
+template <int DT>
+__device__ bool density_again(const DevGrid& g, const DartParams& prm, float x, float y, float z) {
+    const float o[3] = {x, y, z};
+    float f[3], w[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float p = position_exact(prm, a, o[a]);
+        // p - wo = s + t (two-difference, then wo's second float)
+        const float s = __fsub_rn(p, prm.wo_hi[a]);
+        const float bb = __fsub_rn(p, s);
+        const float e = __fadd_rn(__fsub_rn(p, __fadd_rn(s, bb)), __fsub_rn(bb, prm.wo_hi[a]));
+        const float t = __fsub_rn(e, prm.wo_lo[a]);
+        // times 1 / h = inv_h_f + inv_h_lo
+        const float q = __fmul_rn(s, prm.inv_h_f);
+        const float r = __fmaf_rn(t, prm.inv_h_f, __fmaf_rn(s, prm.inv_h_lo, __fmaf_rn(s, prm.inv_h_f, -q)));
+        f[a] = floorf(q);
+        w[a] = __fadd_rn(__fsub_rn(q, f[a]), r);  // outside [0, 1): undecided
     }
-    const double dx = ((double)p[0] - prm.wo[0]) / prm.h;
-    const double dy = ((double)p[1] - prm.wo[1]) / prm.h;
-    const double dz = ((double)p[2] - prm.wo[2]) / prm.h;
-    return !(sample_exact(g, dx, dy, dz) < prm.cutoff);
+    const DartCell c = {w[0], w[1], w[2], cell_record(g, (int)f[0], (int)f[1], (int)f[2])};
+    float v[8];
+    ld_cell<DT>(g.data, c.rec, v);
+    const int d = density_test<DT>(c, v, prm.index_err2, prm.cutoff);
+    return d == 2 ? !(density_exact(g, prm, x, y, z) < prm.cutoff) : d == 1;
+}
+
+template <int DT>
+__device__ __forceinline__ bool density_passes(const DevGrid& g, const DartParams& prm, const DartCell& c,
+                                               const float v[8], const float x[3]) {
+    const int d = density_test<DT>(c, v, prm.index_err, prm.cutoff);
+    return d == 2 ? density_again<DT>(g, prm, x[0], x[1], x[2]) : d == 1;
 }
 
 // |a - b|^2 < m2 as the reference decides it (double arithmetic on float
 // coordinates), with an FP32 fast path outside a 2^-18 relative band.
+__device__ __noinline__ bool closer_fp64(float ax, float ay, float az, const float* b, float m2) {
+    const double ex = __dsub_rn((double)ax, (double)b[0]);
+    const double ey = __dsub_rn((double)ay, (double)b[1]);
+    const double ez = __dsub_rn((double)az, (double)b[2]);
+    const double e2 = __dadd_rn(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)), __dmul_rn(ez, ez));
+    return e2 < (double)m2;
+}
 __device__ __forceinline__ bool closer(const float* a, const float* b, float m2) {
     const float dx = a[0] - b[0], dy = a[1] - b[1], dz = a[2] - b[2];
     const float d2 = dx * dx + dy * dy + dz * dz;
     if (d2 < m2 * (1.f - 3.814697265625e-6f)) return true;
     if (d2 > m2 * (1.f + 3.814697265625e-6f)) return false;
-    const double ex = __dsub_rn((double)a[0], (double)b[0]);
-    const double ey = __dsub_rn((double)a[1], (double)b[1]);
-    const double ez = __dsub_rn((double)a[2], (double)b[2]);
-    const double e2 = __dadd_rn(__dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)), __dmul_rn(ez, ez));
-    return e2 < (double)m2;
+    return closer_fp64(a[0], a[1], a[2], b, m2);
 }
 
-// One MT19937 state block: new[i] = f(old[i], old[i+1], x) with x =
-// old[i+397] for i < 227 and new[i-227] after, i = 623 taking new[0] as its
-// next. Word i >= 227 depends only on word i - 227, so thread t < 227
-// computes the chain t, t + 227, t + 454 alone; word 623 (from new[0] and
-// new[396]) is left to the one thread that uses it. t >= 227 does nothing.
-__device__ __forceinline__ void mt_twist_block(const uint32_t* cur, uint32_t* nxt, int t) {
-    if (t < 0 || t >= 227) return;
-    uint32_t x = mt_twist_word(cur[t], cur[t + 1], cur[t + kMtM]);
-    nxt[t] = x;
-    x = mt_twist_word(cur[t + 227], cur[t + 228], x);
-    nxt[t + 227] = x;
-    if (t < 169) nxt[t + 454] = mt_twist_word(cur[t + 454], cur[t + 455], x);
+// The next chunk's words nxt[0..kBlocks * 624) after this chunk's cur, a state
+// block of 624 at a time. Word i of a block is made of the words 624, 623 and
+// 227 before it, so thread t < 227 makes the words t, t + 227 and t + 454 (the
+// last by 170 threads) from the block before and its own; only word 623 needs
+// another, the block's first, and makes it for itself. The kDartTwisters
+// threads that call it meet at barrier 1 after each block.
+template <int kBlocks>
+__device__ __forceinline__ void mt_next_chunk(const uint32_t* cur, uint32_t* nxt, int t) {
+    const uint32_t* prev = cur + (kBlocks - 1) * kMtN;
+#pragma unroll 1
+    for (int k = 0; k < kBlocks; ++k) {
+        uint32_t* out = nxt + k * kMtN;
+        if (t < kMtN - kMtM) {
+            const bool third = t < kMtN - 2 * (kMtN - kMtM);
+            const uint32_t a0 = prev[t], b0 = prev[t + 1], c0 = prev[t + kMtM];
+            const uint32_t a1 = prev[t + 227], b1 = prev[t + 228];
+            uint32_t a2 = 0u, b2 = 0u;
+            if (third) {
+                a2 = prev[t + 454];
+                b2 = t + 455 < kMtN ? prev[t + 455] : mt_twist_word(prev[0], prev[1], prev[kMtM]);
+            }
+            uint32_t x = mt_twist_word(a0, b0, c0);
+            out[t] = x;
+            x = mt_twist_word(a1, b1, x);
+            out[t + 227] = x;
+            if (third) out[t + 454] = mt_twist_word(a2, b2, x);
+        }
+        prev = out;
+        asm volatile("bar.sync 1, %0;" ::"n"(kDartTwisters) : "memory");
+    }
+}
+
+// Cell coordinate along axis a, clamped to the grid; monotonic in x (every
+// step rounds monotonically), so the points within r of x lie in the cells
+// from that of x - r to that of x + r.
+__device__ __forceinline__ int dart_cell(const DartParams& prm, int a, float x, float inv, int n) {
+    return min(max((int)((x - prm.bb_hi[a]) * inv), 0), n - 1);
+}
+__device__ __forceinline__ int hint_cell(const DartParams& prm, const float p[3]) {
+    return (dart_cell(prm, 2, p[2], prm.hint_inv[2], kDartHint) * kDartHint +
+            dart_cell(prm, 1, p[1], prm.hint_inv[1], kDartHint)) *
+               kDartHint +
+           dart_cell(prm, 0, p[0], prm.hint_inv[0], kDartHint);
 }
 
 // The reference's radius update: minDist^2 *= pcSize / expectedSize, in
 // double, rounded back to float.
-__device__ __forceinline__ void radius_update(float& m2, int pc, uint32_t expected) {
+__device__ __noinline__ void radius_update(float& m2, int pc, uint32_t expected) {
     const double ratio = (double)pc / (double)expected;
     m2 = __double2float_rn(__dmul_rn((double)m2, ratio));
 }
 
-__global__ void __launch_bounds__(kDartThreads, 4) k_dart(DevGrid g, DartParams prm, const uint32_t* __restrict__ expected,
-                                                          float* __restrict__ out_pts, int32_t* __restrict__ out_count,
-                                                          float* __restrict__ out_last_m2) {
-    __shared__ uint32_t mt_a[kMtN], mt_b[kMtN];
-    __shared__ float cand[kDartBlock][3];
-    __shared__ uint8_t dens_ok[kDartBlock], hit[kDartBlock];
-    extern __shared__ float acc_pts[];  // hard_limit x 3
-    __shared__ int s_pc, s_done;
-    __shared__ float s_m2, s_last;
+// Whether one of the two points of the candidate's hint cell is certainly
+// closer; x: its offsets from bbmin.
+__device__ __forceinline__ bool hinted(const ushort2* hint, const float* acc, const DartParams& prm, const float x[3],
+                                       float hint_m2) {
+    const float p[3] = {x[0] + prm.bb_hi[0], x[1] + prm.bb_hi[1], x[2] + prm.bb_hi[2]};
+    const ushort2 h = hint[hint_cell(prm, p)];
+    auto near = [&](int q) {
+        const float dx = p[0] - acc[3 * q], dy = p[1] - acc[3 * q + 1], dz = p[2] - acc[3 * q + 2];
+        return dx * dx + dy * dy + dz * dz < hint_m2;
+    };
+    return (h.x != kNoPoint && near(h.x)) || (h.y != kNoPoint && near(h.y));
+}
+
+// Two warps may do this to one cell at once: whichever entries remain, each
+// is an accepted point.
+__device__ __forceinline__ void add_hint(ushort2& h, int q) { h = make_ushort2((unsigned short)q, h.x); }
+
+// Sizes and dynamic shared memory of a k_dart instance (kBlocks MT19937 state
+// blocks a chunk).
+template <int kBlocks>
+struct DartShared {
+    static constexpr int kWords = kBlocks * kMtN;
+    static constexpr int kCand = kWords / 3;  // candidates a chunk (3 draws each)
+    static constexpr int kSurv = (kCand + 1023) / 1024 * 32;
+    static_assert(kCand % 64 == 0, "groups of 64 are claimed");
+    uint32_t words[2][kWords];
+    uint32_t surv[kSurv];   // survivors, a bit per candidate of the chunk
+    uint16_t queue[kCand];  // candidates left by the hint test, in any order
+    uint16_t head[kDartGrid * kDartGrid * kDartGrid];
+    ushort2 hint[kDartHint * kDartHint * kDartHint];  // the last two points found, the latest in x
+    int claim, queued, pc, done;
+    float m2, last;
+    // then hard_limit x 3 floats (accepted points) and hard_limit uint16 (the
+    // next point of the same cell)
+};
+
+template <int DT, int kThreads, int kBlocks>
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_dart(DevGrid g, DartParams prm, const uint32_t* __restrict__ expected,
+                                                                    float* __restrict__ out_pts,
+                                                                    int32_t* __restrict__ out_count,
+                                                                    float* __restrict__ out_last_m2) {
+    static_assert(kThreads > kDartTwisters && kThreads <= 1024, "the last warps make the next words");
+    using Shared = DartShared<kBlocks>;
+    constexpr int kWarps = kThreads / 32;
+    extern __shared__ __align__(16) uint8_t dart_smem[];
+    Shared& sh = *reinterpret_cast<Shared*>(dart_smem);
+    float* acc = reinterpret_cast<float*>(dart_smem + sizeof(Shared));
+    uint16_t* link = reinterpret_cast<uint16_t*>(acc + 3 * prm.hard_limit);
 
     const int it = prm.first_iter + (int)blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
+        // the seeded state stands before the first chunk
+        uint32_t* st = sh.words[1] + Shared::kWords - kMtN;
         uint32_t x = prm.seed_base + (uint32_t)it;
-        mt_a[0] = x;
+        st[0] = x;
+#pragma unroll 1
         for (int k = 1; k < kMtN; ++k) {
             x = mt_init_word(x, (uint32_t)k);
-            mt_a[k] = x;
+            st[k] = x;
         }
-        s_pc = 0;
-        s_done = 0;
-        s_m2 = prm.min_dist_sq0;
-        s_last = prm.min_dist_sq0;
+        sh.pc = 0;
+        sh.done = 0;
+        sh.m2 = prm.min_dist_sq0;
+        sh.last = prm.min_dist_sq0;
+    } else {
+#pragma unroll 1
+        for (int k = tid - 1; k < kDartGrid * kDartGrid * kDartGrid; k += kThreads - 1) sh.head[k] = kNoPoint;
+#pragma unroll 1
+        for (int k = tid - 1; k < kDartHint * kDartHint * kDartHint; k += kThreads - 1)
+            sh.hint[k] = make_ushort2(kNoPoint, kNoPoint);
+        for (int k = tid - 1; k < Shared::kSurv; k += kThreads - 1) sh.surv[k] = 0u;
     }
     __syncthreads();
-    uint32_t* cur = mt_a;
-    uint32_t* nxt = mt_b;
-    mt_twist_block(cur, nxt, tid);
+    const int twister = tid - (kThreads - kDartTwisters);
+    if (twister >= 0) mt_next_chunk<kBlocks>(sh.words[1], sh.words[0], twister);
+    // candidate n updates the radius before its tests when (n + 1) % batch == 0:
+    // the next such n, and which update it is
+    uint64_t boundary = prm.batch - 1u;
+    uint32_t update = 0;
+    if (tid == 0) {
+        sh.claim = 0;
+        sh.queued = 0;
+        if (boundary == 0u) radius_update(sh.m2, 0, expected[0]);
+    }
     __syncthreads();
-    for (uint32_t base = 0; base < prm.scatter_count; base += kDartBlock) {
-        if (s_done) break;
-        // the block's words (twisted during the previous walk) become current
-        {
-            uint32_t* t = cur;
-            cur = nxt;
-            nxt = t;
+    uint64_t chunk = 0, n0 = 0;  // first candidates of the chunk and of the range
+    int buf = 0;
+    while (n0 < prm.scatter_count) {
+        if (n0 == boundary) {  // its update was made where the last range ended
+            boundary += prm.batch;
+            ++update;
         }
-        // 1. positions and densities of this block's candidates; a radius
-        // update at the block's first candidate is applied alongside by an
-        // idle thread (the accepted count is final: the last walk is done)
-        if (tid < kDartBlock) {
-            // the last word of the block (read only by this candidate, and by
-            // the next twist after a barrier)
-            if (tid == kDartBlock - 1) cur[kMtN - 1] = mt_twist_word(nxt[kMtN - 1], cur[0], cur[396]);
-            const uint32_t n = base + (uint32_t)tid;
-            bool ok = false;
-            if (n < prm.scatter_count) {
-                float p[3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    const float u = mt_canonical_float(mt_temper(cur[3 * tid + a]));
-                    // newPos = float(double(float(u * size)) + bbox.min)
-                    p[a] = __double2float_rn(__dadd_rn((double)__fmul_rn(u, prm.bbsize[a]), prm.bbmin[a]));
-                    cand[tid][a] = p[a];
-                }
-                ok = density_passes(g, p, prm);
-            }
-            dens_ok[tid] = ok;
-        } else if (tid == kDartThreads - 1 && (base + 1u) % prm.batch == 0u) {
-            radius_update(s_m2, s_pc, expected[base / prm.batch]);
+        const uint32_t* cur = sh.words[buf];
+        const uint64_t chunk_end = min(chunk + (uint64_t)Shared::kCand, (uint64_t)prm.scatter_count);
+        const uint64_t n1 = min(chunk_end, boundary);
+        const int j0 = (int)(n0 - chunk), j1 = (int)(n1 - chunk);
+        const int p0 = sh.pc;
+        const float m2 = sh.m2;
+        // r covers sqrt(m2) and the rounding of x -+ r
+        const float root = sqrtf(m2), r = fmaf(root, 1.00001f, prm.cell_slack);
+        // 1. the next chunk's words; density and hint tests. The hint tests
+        // take x + bbmin in plain FP32, off by less than cell_slack / 4 per
+        // axis, which moves a squared distance near m2 by less than root *
+        // cell_slack: below hint_m2 the exact test says the same, and whoever
+        // is not below it is left for the exact one
+        if (twister >= 0 && j0 == 0 && chunk_end < prm.scatter_count)
+            mt_next_chunk<kBlocks>(cur, sh.words[buf ^ 1], twister);
+        const float hint_m2 = m2 * (1.f - 7.62939453125e-6f) - 2.f * prm.cell_slack * root;
+        for (;;) {
+            int j = 0;
+            if (lane == 0) j = atomicAdd(&sh.claim, 64);
+            j = __shfl_sync(0xffffffffu, j, 0) + (j0 & ~63);
+            if (j >= j1) break;
+            // two groups at a time: both record loads are in flight together
+            float xa[3], xb[3], va[8], vb[8];
+            const int ja = j + lane, jb = ja + 32;
+            candidate_offsets(prm, cur + 3 * ja, xa);
+            const DartCell ca = candidate_cell(g, prm, xa);
+            ld_cell<DT>(g.data, ca.rec, va);
+            candidate_offsets(prm, cur + 3 * jb, xb);
+            const DartCell cb = candidate_cell(g, prm, xb);
+            ld_cell<DT>(g.data, cb.rec, vb);
+            const bool pa = ja >= j0 && ja < j1 && density_passes<DT>(g, prm, ca, va, xa);
+            const bool pb = jb >= j0 && jb < j1 && density_passes<DT>(g, prm, cb, vb, xb);
+            const bool la = pa && !hinted(sh.hint, acc, prm, xa, hint_m2), lb = pb && !hinted(sh.hint, acc, prm, xb, hint_m2);
+            const unsigned ma = __ballot_sync(0xffffffffu, la), mb = __ballot_sync(0xffffffffu, lb);
+            if ((ma | mb) == 0u) continue;
+            const unsigned below = (1u << lane) - 1u;
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&sh.queued, __popc(ma) + __popc(mb));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (la) sh.queue[at + __popc(ma & below)] = (uint16_t)ja;
+            if (lb) sh.queue[at + __popc(ma) + __popc(mb & below)] = (uint16_t)jb;
         }
         __syncthreads();
-        // 2-3. segments between radius updates (candidate n updates before
-        // its tests when (n + 1) % batch == 0): one per block but for the
-        // blocks that hold a radius update past their first candidate
-        int j0 = 0;
-        const int jend = (int)min((uint32_t)kDartBlock, prm.scatter_count - base);
-        while (j0 < jend && !s_done) {
-            // next boundary after j0: the smallest n > base + j0 with
-            // (n + 1) % batch == 0
-            const uint32_t m = base + (uint32_t)j0 + 1u;
-            const uint64_t nb = ((uint64_t)(m + 1u) + prm.batch - 1u) / prm.batch * prm.batch - 1u;
-            const int j1 = (int)min((uint64_t)jend, nb - base);
-            if (j0 > 0) {
-                // the update belongs to candidate j0, a boundary
-                if (tid == 0) radius_update(s_m2, s_pc, expected[(base + j0) / prm.batch]);
-                __syncthreads();
+        // 2. the accepted points near each candidate left; lane k of a warp
+        // holds the position of its k-th
+        const int nq = sh.queued;
+#pragma unroll 1
+        for (int e0 = 0; e0 < nq; e0 += kThreads) {
+            const int e = e0 + warp + kWarps * lane;
+            int jj = 0;
+            float p[3] = {0.f, 0.f, 0.f};
+            if (e < nq) {
+                jj = sh.queue[e];
+                candidate_position(prm, cur + 3 * jj, p);
             }
-            const int p0 = s_pc;
-            const float m2 = s_m2;
-            // 2. survivors of the points accepted before the segment
-            for (int j = j0 + warp; j < j1; j += kDartWarps) {
-                bool h = false;
-                if (dens_ok[j]) {
-                    for (int q0 = 0; q0 < p0 && !h; q0 += 32) {
-                        const int q = q0 + lane;
-                        const bool c = q < p0 && closer(cand[j], acc_pts + 3 * q, m2);
-                        h = __any_sync(0xffffffffu, c);
-                    }
+            const int mine = __popc(__ballot_sync(0xffffffffu, e < nq));
+#pragma unroll 1
+            for (int k = 0; k < mine; ++k) {
+                const float q[3] = {__shfl_sync(0xffffffffu, p[0], k), __shfl_sync(0xffffffffu, p[1], k),
+                                    __shfl_sync(0xffffffffu, p[2], k)};
+                const int jk = __shfl_sync(0xffffffffu, jj, k);
+                int lo[3], hi[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    lo[a] = dart_cell(prm, a, q[a] - r, prm.cell_inv[a], kDartGrid);
+                    hi[a] = dart_cell(prm, a, q[a] + r, prm.cell_inv[a], kDartGrid);
                 }
-                if (lane == 0) hit[j] = h;
+                const int cells = (hi[0] - lo[0] + 1) * (hi[1] - lo[1] + 1) * (hi[2] - lo[2] + 1);
+                unsigned hits = 0u;
+                int near = 0;
+                if (cells >= p0) {  // few points yet: all of them
+#pragma unroll 1
+                    for (int i0 = 0; i0 < p0 && !hits; i0 += 32) {
+                        near = i0 + lane;
+                        hits = __ballot_sync(0xffffffffu, near < p0 && closer(q, acc + 3 * near, m2));
+                    }
+                } else {
+                    // 4 x 4 x 2 cells at a time, a lane each
+                    const int lx = lane & 3, ly = (lane >> 2) & 3, lz = lane >> 4;
+#pragma unroll 1
+                    for (int z = lo[2]; z <= hi[2] && !hits; z += 2)
+#pragma unroll 1
+                        for (int y = lo[1]; y <= hi[1] && !hits; y += 4)
+#pragma unroll 1
+                            for (int x = lo[0]; x <= hi[0] && !hits; x += 4) {
+                                bool h = false;
+                                if (x + lx <= hi[0] && y + ly <= hi[1] && z + lz <= hi[2]) {
+                                    near = sh.head[((z + lz) * kDartGrid + y + ly) * kDartGrid + x + lx];
+                                    while (near != kNoPoint && !(h = closer(q, acc + 3 * near, m2))) near = link[near];
+                                }
+                                hits = __ballot_sync(0xffffffffu, h);
+                            }
+                }
+                if (hits) {
+                    if (lane == __ffs(hits) - 1) add_hint(sh.hint[hint_cell(prm, q)], near);
+                } else if (lane == 0) {
+                    atomicOr(&sh.surv[jk >> 5], 1u << (jk & 31));
+                }
             }
-            __syncthreads();
-            // 3. walk the survivors in order (warp 0; lane 0 accepts); after
-            // the block's last segment, warps 1-8 twist the next block's
-            // words meanwhile (they read this block's words, which the walk
-            // does not touch, and overwrite the previous block's)
-            if (warp == 0) {
-                for (int c0 = j0; c0 < j1; c0 += 32) {
-                    const int j = c0 + lane;
-                    const unsigned live = __ballot_sync(0xffffffffu, j < j1 && dens_ok[j] && !hit[j]);
-                    if (lane == 0) {
-                        unsigned mk = live;
-                        while (mk && !s_done) {
-                            const int jj = c0 + __ffs(mk) - 1;
-                            mk &= mk - 1;
-                            bool h = false;
-                            for (int q = p0; q < s_pc && !h; ++q) h = closer(cand[jj], acc_pts + 3 * q, m2);
-                            if (h) continue;
-                            const int k = s_pc;
-                            acc_pts[3 * k] = cand[jj][0];
-                            acc_pts[3 * k + 1] = cand[jj][1];
-                            acc_pts[3 * k + 2] = cand[jj][2];
-                            s_pc = k + 1;
-                            s_last = m2;
-                            // the reference stops at the next candidate once
-                            // more than target points are accepted
-                            if (s_pc > (int)prm.target || s_pc >= (int)prm.hard_limit) s_done = 1;
+        }
+        __syncthreads();
+        // 3. the walk
+        if (warp == 0) {
+            int pc = p0;
+            bool done = false;
+            float last = sh.last;
+#pragma unroll 1
+            for (int half = 0; half < Shared::kSurv && !done; half += 32) {
+                const uint32_t mine = sh.surv[half + lane];
+                sh.surv[half + lane] = 0u;
+                unsigned some = __ballot_sync(0xffffffffu, mine != 0u);
+                while (some && !done) {
+                    const int k = __ffs(some) - 1;
+                    some &= some - 1;
+                    uint32_t bits = __shfl_sync(0xffffffffu, mine, k);
+                    float p[3] = {0.f, 0.f, 0.f};
+                    if ((bits >> lane) & 1u) candidate_position(prm, cur + 3 * (32 * (half + k) + lane), p);
+                    while (bits && !done) {
+                        const int b = __ffs(bits) - 1;
+                        bits &= bits - 1;
+                        const float q[3] = {__shfl_sync(0xffffffffu, p[0], b), __shfl_sync(0xffffffffu, p[1], b),
+                                            __shfl_sync(0xffffffffu, p[2], b)};
+                        bool h = false;
+                        for (int i0 = p0; i0 < pc && !h; i0 += 32)
+                            h = __any_sync(0xffffffffu, i0 + lane < pc && closer(q, acc + 3 * (i0 + lane), m2));
+                        if (h) continue;
+                        if (lane == 0) {
+                            acc[3 * pc] = q[0];
+                            acc[3 * pc + 1] = q[1];
+                            acc[3 * pc + 2] = q[2];
+                            const int c = (dart_cell(prm, 2, q[2], prm.cell_inv[2], kDartGrid) * kDartGrid +
+                                           dart_cell(prm, 1, q[1], prm.cell_inv[1], kDartGrid)) *
+                                              kDartGrid +
+                                          dart_cell(prm, 0, q[0], prm.cell_inv[0], kDartGrid);
+                            link[pc] = sh.head[c];
+                            sh.head[c] = (uint16_t)pc;
+                            add_hint(sh.hint[hint_cell(prm, q)], pc);
                         }
+                        __syncwarp();
+                        ++pc;
+                        last = m2;
+                        // the reference stops at the next candidate once
+                        // more than target points are accepted
+                        done = pc > (int)prm.target || pc >= (int)prm.hard_limit;
                     }
-                    __syncwarp();
                 }
-            } else if (j1 == jend) {
-                mt_twist_block(cur, nxt, tid - 32);
             }
-            __syncthreads();
-            j0 = j1;
+            if (lane == 0) {
+                sh.pc = pc;
+                sh.last = last;
+                sh.done = done;
+                sh.claim = 0;
+                sh.queued = 0;
+                if (n1 == boundary && n1 < prm.scatter_count) radius_update(sh.m2, pc, expected[update]);
+            }
+        }
+        __syncthreads();
+        if (sh.done) break;
+        n0 = n1;
+        if (n1 == chunk_end) {
+            chunk = n1;
+            buf ^= 1;
         }
     }
-    __syncthreads();
-    const int pc = s_pc;
+    const int pc = sh.pc;
     float* dst = out_pts + (size_t)blockIdx.x * prm.hard_limit * 3;
-    for (int k = tid; k < 3 * pc; k += kDartThreads) dst[k] = acc_pts[k];
+    for (int k = tid; k < 3 * pc; k += kThreads) dst[k] = acc[k];
     if (tid == 0) {
         out_count[blockIdx.x] = pc;
-        out_last_m2[blockIdx.x] = s_last;
+        out_last_m2[blockIdx.x] = sh.last;
     }
+}
+
+template <int DT, int kThreads, int kBlocks>
+cudaError_t launch_dart_t(const DevGrid& g, const DartParams& prm, int n_iter, const uint32_t* expected, float* out_pts,
+                          int32_t* out_count, float* out_last_m2, cudaStream_t st) {
+    const size_t smem = sizeof(DartShared<kBlocks>) + (3 * sizeof(float) + sizeof(uint16_t)) * (size_t)prm.hard_limit;
+    const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k_dart<DT, kThreads, kBlocks>));
+    if (e != cudaSuccess) return e;
+    k_dart<DT, kThreads, kBlocks><<<n_iter, kThreads, smem, st>>>(g, prm, expected, out_pts, out_count, out_last_m2);
+    ++g_launch_counter;
+    return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_dart(const DevGrid& g, const DartParams& prm, int n_iter, const uint32_t* expected, float* out_pts,
+cudaError_t launch_dart(const DevGrid& g, DartParams prm, int n_iter, const uint32_t* expected, float* out_pts,
                         int32_t* out_count, float* out_last_m2, cudaStream_t st) {
     if (n_iter <= 0) return cudaSuccess;
-    const size_t smem = sizeof(float) * 3 * prm.hard_limit;
-    if (smem > 32 * 1024) {  // with the static arrays, past the default 48 KB
-        const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k_dart));
-        if (e != cudaSuccess) return e;
+    float extent = 0.f;
+    for (int a = 0; a < 3; ++a) {
+        prm.bb_hi[a] = (float)prm.bbmin[a];
+        prm.bb_lo[a] = (float)(prm.bbmin[a] - (double)prm.bb_hi[a]);
+        // what position_exact leaves out besides the rounding of e + lo: the
+        // part of bbmin below hi + lo and the double sum's own rounding
+        prm.bb_err[a] = (float)((std::fabs(prm.bbmin[a]) + (double)prm.bbsize[a]) * 1.4210854715202004e-14);  // 2^-46
+        prm.wo_hi[a] = (float)prm.wo[a];
+        prm.wo_lo[a] = (float)(prm.wo[a] - (double)prm.wo_hi[a]);
+        prm.cell_inv[a] = (float)kDartGrid / prm.bbsize[a];
+        prm.hint_inv[a] = (float)kDartHint / prm.bbsize[a];
+        extent = std::max(extent, std::fabs(prm.bb_hi[a]) + prm.bbsize[a]);
     }
-    k_dart<<<n_iter, kDartThreads, smem, st>>>(g, prm, expected, out_pts, out_count, out_last_m2);
-    ++g_launch_counter;
-    return cudaGetLastError();
+    prm.inv_h_lo = (float)(1.0 / prm.h - (double)prm.inv_h_f);
+    prm.cell_slack = extent * 1e-6f;
+    // As long as every iteration gets an SM of its own, the chain of its ranges
+    // is what takes the time: 1024 threads and chunks of 3328 candidates shorten
+    // it; past that, two CTAs of 512 threads with chunks of 1664 on an SM fill
+    // each other's waits.
+    int sms = 0, dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    auto go = [&](auto launch) { return launch(g, prm, n_iter, expected, out_pts, out_count, out_last_m2, st); };
+    if (n_iter <= sms)
+        return g.dtype == 1   ? go(launch_dart_t<1, 1024, 16>)
+               : g.dtype == 2 ? go(launch_dart_t<2, 1024, 16>)
+                              : go(launch_dart_t<0, 1024, 16>);
+    return g.dtype == 1   ? go(launch_dart_t<1, 512, 8>)
+           : g.dtype == 2 ? go(launch_dart_t<2, 512, 8>)
+                          : go(launch_dart_t<0, 512, 8>);
 }
 
 }  // namespace lg

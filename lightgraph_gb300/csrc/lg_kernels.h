@@ -238,13 +238,20 @@ struct DartParams {
     double bbmin[3];  // active-voxel bbox, world space
     float bbsize[3];
     double wo[3], h;  // the grid's world origin and voxel size
-    float wo_f[3], inv_h_f;  // the same in FP32 (fast path)
-    float index_err;         // bound of the FP32 index-position error (voxels)
+    // FP32 fast path: index-space position of an offset x from bbmin = x *
+    // inv_h_f + index0, off by at most index_err voxels
+    float inv_h_f, index0[3], index_err;
+    float index_err2;  // of the index position formed from two-float sums
+    // made by launch_dart: bbmin as two floats and what that leaves out, wo and
+    // 1 / h as two floats (the first of 1 / h is inv_h_f), cells per world unit
+    // of the point and hint grids, rounding slack of a radius
+    float bb_hi[3], bb_lo[3], bb_err[3], wo_hi[3], wo_lo[3], inv_h_lo;
+    float cell_inv[3], hint_inv[3], cell_slack;
 };
 // expected: the expected sizes at the scatter_count / batch radius updates;
 // out_pts: n_iter x hard_limit x 3 floats; out_last_m2: the squared minimum
 // distance of each iteration's last accepted point.
-cudaError_t launch_dart(const DevGrid& g, const DartParams& prm, int n_iter, const uint32_t* expected, float* out_pts,
+cudaError_t launch_dart(const DevGrid& g, DartParams prm, int n_iter, const uint32_t* expected, float* out_pts,
                         int32_t* out_count, float* out_last_m2, cudaStream_t st);
 
 // Environment map CDFs (FP64 prefix sums)

@@ -59,3 +59,35 @@ def test_scatter_graphs_connects_like_oracle(gpu_ctx):
         oadj, ne = o.build_graph(pts[i], float(r2[i]), 12)
         assert ne > 0
         assert np.array_equal(adj[i].astype(bool), oadj.astype(bool))
+
+
+@pytest.mark.parametrize("kw, dtype, origin", [
+    (dict(scatter_count=1663, n_estimates=3), 0, (0, 0, 0)),            # below one chunk of 1664 candidates
+    (dict(scatter_count=1665, n_estimates=1665), 0, (0, 0, 0)),         # one past it; a radius update per candidate
+    (dict(scatter_count=2 * 1664, n_estimates=7), 1, (0, 0, 0)),        # whole chunks; updates inside them
+    (dict(scatter_count=30000, n_estimates=18, target_size=5, hard_limit=7), 0, (0, 0, 0)),  # ends early
+    (dict(scatter_count=60000, target_size=4000, hard_limit=4096, min_dist_mult=0.01), 2, (0, 0, 0)),  # most points
+    (dict(scatter_count=20000, min_dist_mult=3.0), 0, (0, 0, 0)),       # a radius over the whole box
+    (dict(scatter_count=40000), 0, (3.7, -120.3, 1000.1)),              # bbmin far from a float; coarse index space
+])
+def test_scatter_points_chunk_edges(gpu_ctx, kw, dtype, origin):
+    """Candidate counts around a chunk, radius updates inside and at its ends,
+    the smallest and largest point limits, storage types and a far world
+    origin: the oracle's points, bit for bit."""
+    sc = scenes.small(n_points=16, res=64)
+    v = sc.density.values
+    if dtype == 1:
+        v = v.astype(np.float16).astype(np.float32)
+    elif dtype == 2:
+        v = (v.view(np.uint32) & np.uint32(0xFFFF0000)).view(np.float32)  # exactly representable in BF16
+    sc.density.values = np.ascontiguousarray(v)
+    sc.density.world_origin = origin
+    scenes.load_into(gpu_ctx, sc, dtype)
+    opts = lgm.scatter_opts(**kw)
+    pts, r2 = gpu_ctx.scatter_points(11, 3, opts)
+    opt, ocnt, om2 = po.scatter_points(sc.density, opts, 11, 3)
+    for i in range(3):
+        assert len(pts[i]) == ocnt[i]
+        assert np.array_equal(pts[i].view(np.uint32), opt[i, :ocnt[i]].view(np.uint32))
+        # (an expected size of 0 makes the radius NaN, on both sides)
+        assert np.array_equal(np.float32(r2[i]), connect_r2(om2[i], opts.connect_mult), equal_nan=True)
