@@ -669,11 +669,16 @@ lg_status Ctx::load_graphs(int n_graphs, const float* points, const int64_t* off
 
 lg_status Ctx::build_edges() {
     Ctx* ctx = this;
-    CK(launch_candidates(d_pts.as<float>(), d_graphs.as<GraphInfo>(), d_pt_graph.as<int32_t>(), n_points,
-                         d_cand.as<uint16_t>(), d_cand_cnt.as<int32_t>(), st), "edge candidates");
-    CK(launch_greedy(d_pts.as<float>(), d_graphs.as<GraphInfo>(), n_graphs, max_n, d_cand.as<uint16_t>(),
-                     d_cand_cnt.as<int32_t>(), max_connect, d_edges.as<int2>(), d_edge_cnt.as<int32_t>(), st),
-       "greedy connect");
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "device query");
+    PairScratch ps{};
+    if (edge_sweeps(max_n, n_points, max_connect, sms)) {
+        CK(d_pairs.reserve(pair_scratch_bytes(n_points, n_graphs)), "pair scratch alloc");
+        ps = pair_scratch(d_pairs.p, n_points);
+    }
+    CK(launch_edges(d_pts.as<float>(), d_graphs.as<GraphInfo>(), d_pt_graph.as<int32_t>(), n_graphs, max_n, n_points,
+                    max_connect, d_cand.as<uint16_t>(), d_cand_cnt.as<int32_t>(), ps, d_edges.as<int2>(),
+                    d_edge_cnt.as<int32_t>(), sms, st), "connect points");
     graphs_built = true;
     return LG_OK;
 }

@@ -23,12 +23,26 @@ struct GraphInfo {
 
 constexpr int kCandCap = 96;  // stored candidate partners per row
 
-cudaError_t launch_candidates(const float* pts, const GraphInfo* graphs, const int32_t* pt_graph,
-                              int64_t n_points, uint16_t* cand, int32_t* cand_cnt,
-                              cudaStream_t st);
-cudaError_t launch_greedy(const float* pts, const GraphInfo* graphs, int n_graphs, int max_n,
-                          const uint16_t* cand, const int32_t* cand_cnt, int max_connect,
-                          int2* edges, int32_t* edge_cnt, cudaStream_t st);
+// Scratch of the edge selection by sweeps: per point kCandCap places for the
+// partners below it, their number, a limit and kPairStateWords words of state;
+// left: two words per graph.
+constexpr int kPairStateWords = 16;
+struct PairScratch {
+    uint16_t* lower;
+    int32_t* lower_cnt;
+    uint32_t* limits;
+    uint32_t* states;
+    int32_t* left;
+};
+size_t pair_scratch_bytes(int64_t n_points, int n_graphs);
+PairScratch pair_scratch(void* p, int64_t n_points);
+// Whether launch_edges uses sweeps, and so the scratch.
+bool edge_sweeps(int max_n, int64_t n_points, int max_connect, int sms);
+// LightGraph::buildGraph for every graph: the edges in (i, j) order and their
+// number per graph.
+cudaError_t launch_edges(const float* pts, const GraphInfo* graphs, const int32_t* pt_graph, int n_graphs, int max_n,
+                         int64_t n_points, int max_connect, uint16_t* cand, int32_t* cand_cnt, const PairScratch& ps,
+                         int2* edges, int32_t* edge_cnt, int sms, cudaStream_t st);
 cudaError_t launch_adjacency(const GraphInfo* graphs, int n_graphs, int max_edges,
                              const int2* edges, const int32_t* edge_cnt, uint8_t* adj,
                              const int64_t* adj_off, cudaStream_t st);
