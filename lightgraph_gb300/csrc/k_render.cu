@@ -268,8 +268,7 @@ __device__ __forceinline__ int clamp_bin(float x, int n) { return min(max((int)x
 // key below 2^31, so the arithmetic is 32-bit; the point light's cube-map
 // coordinates and distance come from approximate reciprocals (the key only
 // decides the order in which rays are marched).
-__device__ __forceinline__ uint32_t ray_key(const RayBin& b, const float p[3], int64_t t) {
-    if (b.kind == 2) return (uint32_t)(b.key_off + (t >> b.shift));
+__device__ __forceinline__ uint32_t ray_key(const RayBin& b, const float p[3]) {
     uint32_t uv;
     float depth;
     if (b.kind == 0) {
@@ -380,7 +379,7 @@ __device__ __forceinline__ uint32_t primary_sample(const DevScene& sc, const Dev
 #pragma unroll
                             for (int k = 0; k < kMaxLights; ++k) {
                                 if (k >= ko.rb.n) break;
-                                const uint32_t key = ray_key(ko.rb.b[k], p, t);
+                                const uint32_t key = ray_key(ko.rb.b[k], p);
                                 ko.keys[k * ko.unit_cap + u] = key;
                                 // lanes filing under the same key share one atomic
                                 const cg::coalesced_group grp = cg::labeled_partition(cg::coalesced_threads(), key);
@@ -653,17 +652,51 @@ __device__ __forceinline__ void shadow_span_samples(const DevGrid& G, const IRay
     }
 }
 
-// One thread per (light k, ordered slot r): the shadow rays of light k (all
-// its samples) from task kRayUnit * order[k * n_units + r / kRayUnit] +
+// The shadow ray srr (clipped to the leaf bbox) marched to its end: tau is its
+// optical depth (kUnit: in units of 1 / scale); returns false if it dropped
+// out.
+template <int DT, bool kUnit>
+__device__ __forceinline__ bool shadow_march(const DevGrid& G, const ShadowMarch& sm, const IRay& srr, uint32_t sub,
+                                             float step1, float inv_step1, uint32_t& n_shadow, float& tau) {
+    const float half_step1 = 0.5f * step1, quarter_step1 = 0.25f * step1;
+    LeafDDA sd;
+    dda_init_bits(sd, srr, G);
+    float sa, sb;
+    tau = 0.f;
+    uint32_t sspan = 0, siter = 0;
+    uint32_t jit = step_seed_shadow(sub);
+    bool sdrop = false;
+    while (!sdrop && next_span(G, sd, sa, sb)) {
+        float sStep = jitter_step(step1, draw_sub(sub, kTagShadowSpan | sspan));
+        ++sspan;
+        // every jittered step is >= 0.75 step1: if that is not
+        // absorbed at sb, sT grows on every iteration up to sb
+        if (!(sb + 0.75f * step1 > sb)) continue;
+        shadow_span_samples<DT, kUnit>(G, srr, step1 * ceilf(sa * inv_step1), sb, half_step1, quarter_step1, sm, sStep,
+                                       jit, siter, tau);
+        sdrop = tau > sm.drop;
+    }
+    n_shadow += siter;
+    return !sdrop;
+}
+
+// Adds a warp's shadow samples to *ctr.
+__device__ __forceinline__ void count_samples(uint32_t n, unsigned long long* ctr) {
+    unsigned long long q = n;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+    if ((threadIdx.x & 31) == 0) atomicAdd(ctr, q);
+}
+
+// One thread per (ordered light, ordered slot r): the shadow rays of the light
+// (all its samples) from task kRayUnit * order[k * n_units + r / kRayUnit] +
 // r % kRayUnit; warps claim 32 consecutive (light, slot) pairs at a time from
 // ctr[2] (zero at launch), so the lanes of a warp march neighbouring rays.
 // ctr[1] accumulates the shadow samples.
-// direct[k * task_cap + t] = albedo * (sum_ls I * T / ns) * w.
-// kEnv = false leaves the environment-light branch out (no light of the
-// scene is an environment light), which frees registers for occupancy.
+// direct[light * task_cap + t] = albedo * (sum_ls I * T / ns) * w.
 // kUnit = sc.smarch.unit: the density scale folded into the march constants
 // (ShadowMarch), one multiply per ray instead of one per sample.
-template <int DT, bool kEnv, bool kUnit>
+template <int DT, bool kUnit>
 __global__ void __launch_bounds__(128, 8) k_shadow(DevScene sc, RayBins rb, const ShadowTask* __restrict__ tasks,
                                                 const int32_t* __restrict__ total_ptr, int64_t task_cap,
                                                 const int32_t* __restrict__ order, float4* __restrict__ direct,
@@ -673,14 +706,13 @@ __global__ void __launch_bounds__(128, 8) k_shadow(DevScene sc, RayBins rb, cons
     const uint64_t per_light = n_units * kRayUnit;
     const DevGrid& G = sc.dens;
     const DevShader& sh = sc.sh;
-    const float step1 = sc.step1;
-    const float inv_step1 = 1.f / step1, half_step1 = 0.5f * step1, quarter_step1 = 0.25f * step1;
+    const float step1 = sc.step1, inv_step1 = 1.f / step1;
     const ShadowMarch& sm = sc.smarch;
     uint32_t n_shadow = 0;
     // each warp claims the next 32 (light, ordered slot) pairs, lights in
     // order, until none are left: the warps stay busy to the end whatever
     // the rays cost (every ray's result goes to its own slot)
-    const uint64_t n_slots = (uint64_t)sc.n_lights * per_light;
+    const uint64_t n_slots = (uint64_t)rb.n * per_light;
     const int lane = threadIdx.x & 31;
     for (;;) {
         unsigned long long base = 0;
@@ -701,18 +733,14 @@ __global__ void __launch_bounds__(128, 8) k_shadow(DevScene sc, RayBins rb, cons
         const float4 tk0 = __ldg(reinterpret_cast<const float4*>(tasks + t));
         const uint2 tkw = __ldg(reinterpret_cast<const uint2*>(tasks + t) + 3);
         const float tp[3] = {tk0.x, tk0.y, tk0.z};
-        const DevLight& Lk = sc.lights[k];
+        const int light = rb.b[k].light;
+        const DevLight& Lk = sc.lights[light];
         float lum[3] = {0.f, 0.f, 0.f};
         for (int ls = 0; ls < Lk.samples; ++ls) {
-            const uint32_t sub = shadow_key_from(tkw.x, tkw.y, (uint32_t)k, (uint32_t)ls);
+            const uint32_t sub = shadow_key_from(tkw.x, tkw.y, (uint32_t)light, (uint32_t)ls);
             float ldir[3], I[3], dist;
-            if (kEnv && Lk.type == 2) {
-                env_illuminate(sc.env, Lk, draw_sub(sub, kTagEnvU), draw_sub(sub, kTagEnvV), ldir, I);
-                dist = kInf;
-            } else {
-                const float pw[3] = {tp[0] * G.h + G.wo[0], tp[1] * G.h + G.wo[1], tp[2] * G.h + G.wo[2]};
-                illuminate_shadow(Lk, pw, ldir, I, dist);
-            }
+            const float pw[3] = {tp[0] * G.h + G.wo[0], tp[1] * G.h + G.wo[1], tp[2] * G.h + G.wo[2]};
+            illuminate_shadow(Lk, pw, ldir, I, dist);
             IRay srr;
             make_iray_approx(srr, tp[0], tp[1], tp[2], -ldir[0], -ldir[1], -ldir[2], kDelta * G.inv_h,
                              dist * G.inv_h);
@@ -720,24 +748,8 @@ __global__ void __launch_bounds__(128, 8) k_shadow(DevScene sc, RayBins rb, cons
             // past the last leaf of the ray's light-space bin the walk finds no
             // span: stop it there (spans and samples are unchanged)
             srr.t1 = fminf(srr.t1, fmaxf(shadow_ray_end(rb.b[k], tp), srr.t0));
-            LeafDDA sd;
-            dda_init_bits(sd, srr, G);
-            float sa, sb, tau = 0.f;
-            uint32_t sspan = 0, siter = 0;
-            uint32_t jit = step_seed_shadow(sub);
-            bool sdrop = false;
-            while (!sdrop && next_span(G, sd, sa, sb)) {
-                float sStep = jitter_step(step1, draw_sub(sub, kTagShadowSpan | sspan));
-                ++sspan;
-                // every jittered step is >= 0.75 step1: if that is not
-                // absorbed at sb, sT grows on every iteration up to sb
-                if (!(sb + 0.75f * step1 > sb)) continue;
-                shadow_span_samples<DT, kUnit>(G, srr, step1 * ceilf(sa * inv_step1), sb, half_step1, quarter_step1, sm,
-                                               sStep, jit, siter, tau);
-                sdrop = tau > sm.drop;
-            }
-            n_shadow += siter;
-            if (sdrop) continue;
+            float tau;
+            if (!shadow_march<DT, kUnit>(G, sm, srr, sub, step1, inv_step1, n_shadow, tau)) continue;
             if (kUnit) tau *= sm.scale;
 #pragma unroll
             for (int c = 0; c < 3; ++c) lum[c] += I[c] * __expf(-sh.a[c] * tau);
@@ -748,14 +760,126 @@ __global__ void __launch_bounds__(128, 8) k_shadow(DevScene sc, RayBins rb, cons
         float o[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) o[c] = sh.albedo[c] * (lum[c] * inv_ns) * tw[c];
-        direct[(int64_t)k * task_cap + t] = make_float4(o[0], o[1], o[2], 0.f);
+        direct[(int64_t)light * task_cap + t] = make_float4(o[0], o[1], o[2], 0.f);
     }
-    {
-        unsigned long long q = n_shadow;
+    count_samples(n_shadow, ctr + 1);
+}
+
+// --- environment lights ------------------------------------------------------
+
+// Order key of sample ls of environment light k for the task at t.
+__device__ __forceinline__ uint32_t env_key(const DevScene& sc, const EnvOrder& eo, const ShadowTask* tasks, int64_t t,
+                                            int k, int ls) {
+    const float4 tk0 = __ldg(reinterpret_cast<const float4*>(tasks + t));
+    const uint2 tkw = __ldg(reinterpret_cast<const uint2*>(tasks + t) + 3);
+    const uint32_t sub = shadow_key_from(tkw.x, tkw.y, (uint32_t)k, (uint32_t)ls);
+    float d[3], I[3];
+    env_illuminate(sc.env, sc.lights[k], draw_sub(sub, kTagEnvU), draw_sub(sub, kTagEnvV), d, I);
+    // octahedral map of the direction
+    const float inv = __fdividef(1.f, fabsf(d[0]) + fabsf(d[1]) + fabsf(d[2]));
+    float u = d[0] * inv, v = d[1] * inv;
+    if (d[2] < 0.f) {
+        const float fu = (1.f - fabsf(v)) * (u >= 0.f ? 1.f : -1.f);
+        v = (1.f - fabsf(u)) * (v >= 0.f ? 1.f : -1.f);
+        u = fu;
+    }
+    const int nd = 1 << eo.dir_bits, nc = 1 << eo.cell_bits;
+    const uint32_t du = (uint32_t)clamp_bin((u * 0.5f + 0.5f) * (float)nd, nd),
+                   dv = (uint32_t)clamp_bin((v * 0.5f + 0.5f) * (float)nd, nd);
+    const float p[3] = {tk0.x, tk0.y, tk0.z};
+    uint32_t cell = 0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-        if ((threadIdx.x & 31) == 0) atomicAdd(ctr + 1, q);
+    for (int a = 0; a < 3; ++a) {
+        uint32_t c = (uint32_t)clamp_bin((p[a] - eo.lo[a]) * eo.inv_cell, nc);  // at most 8 bits, every third place
+        c = (c | (c << 8)) & 0x0000F00Fu;
+        c = (c | (c << 4)) & 0x000C30C3u;
+        c = (c | (c << 2)) & 0x00249249u;
+        cell |= c << a;
     }
+    return ((spread_bits16(du) | (spread_bits16(dv) << 1)) << (3 * eo.cell_bits)) | cell;
+}
+
+// Counts the keys of one sample of environment light k (counts zeroed first).
+__global__ void __launch_bounds__(256) k_env_keys(DevScene sc, EnvOrder eo, const ShadowTask* __restrict__ tasks,
+                                                  const int32_t* __restrict__ total_ptr, int64_t task_cap, int k, int ls,
+                                                  int32_t* __restrict__ counts) {
+    const int64_t total = min((int64_t)*total_ptr, task_cap);
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t key = env_key(sc, eo, tasks, t, k, ls);
+        eo.keys[t] = key;
+        atomicAdd(counts + key, 1);
+    }
+}
+
+// The counting sort's scatter. Within a key the order is whatever the atomics
+// give; every ray's result goes to its own slot.
+__global__ void __launch_bounds__(256) k_env_scatter(EnvOrder eo, const int32_t* __restrict__ total_ptr, int64_t task_cap,
+                                                     int32_t* __restrict__ offsets) {
+    const int64_t total = min((int64_t)*total_ptr, task_cap);
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x)
+        eo.order[atomicAdd(offsets + eo.keys[t], 1)] = (int32_t)t;
+}
+
+// Samples [s0, s1) of environment light k from every task, in `order` (null:
+// task order), a thread per task; warps claim 32 consecutive places at a time
+// from *claim (zero at launch). The samples' sum goes on in direct between
+// launches and becomes the light's contribution with the last one, with the
+// roundings of one thread taking them in turn.
+template <int DT, bool kUnit>
+__global__ void __launch_bounds__(128, 8) k_shadow_env(DevScene sc, int k, int s0, int s1,
+                                                       const ShadowTask* __restrict__ tasks,
+                                                       const int32_t* __restrict__ total_ptr, int64_t task_cap,
+                                                       const int32_t* __restrict__ order, float4* __restrict__ direct,
+                                                       unsigned long long* __restrict__ ctr,
+                                                       unsigned long long* __restrict__ claim) {
+    const uint64_t total = (uint64_t)min((int64_t)*total_ptr, task_cap);
+    const DevGrid& G = sc.dens;
+    const DevShader& sh = sc.sh;
+    const float step1 = sc.step1, inv_step1 = 1.f / step1;
+    const ShadowMarch& sm = sc.smarch;
+    const DevLight& Lk = sc.lights[k];
+    uint32_t n_shadow = 0;
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(claim, 32ull);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base >= total) break;
+        if (base + lane >= total) continue;
+        const int64_t t = order ? (int64_t)order[base + lane] : (int64_t)(base + lane);
+        const float4 tk0 = __ldg(reinterpret_cast<const float4*>(tasks + t));
+        const uint2 tkw = __ldg(reinterpret_cast<const uint2*>(tasks + t) + 3);
+        float4* out = direct + (int64_t)k * task_cap + t;
+        float lum[3] = {0.f, 0.f, 0.f};
+        if (s0 > 0) {
+            const float4 q = *out;
+            lum[0] = q.x;
+            lum[1] = q.y;
+            lum[2] = q.z;
+        }
+        for (int ls = s0; ls < s1; ++ls) {
+            const uint32_t sub = shadow_key_from(tkw.x, tkw.y, (uint32_t)k, (uint32_t)ls);
+            float ldir[3], I[3];
+            env_illuminate(sc.env, Lk, draw_sub(sub, kTagEnvU), draw_sub(sub, kTagEnvV), ldir, I);
+            IRay srr;
+            make_iray_approx(srr, tk0.x, tk0.y, tk0.z, -ldir[0], -ldir[1], -ldir[2], kDelta * G.inv_h, kInf);
+            if (!clip_to_bbox_flat(G, srr)) continue;  // the reference skips the light sample
+            float tau;
+            if (!shadow_march<DT, kUnit>(G, sm, srr, sub, step1, inv_step1, n_shadow, tau)) continue;
+            if (kUnit) tau *= sm.scale;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) lum[c] += I[c] * __expf(-sh.a[c] * tau);
+        }
+        if (s1 == Lk.samples) {
+            const float inv_ns = __fdividef(1.f, (float)Lk.samples);
+            const float2 w12 = __ldg(reinterpret_cast<const float2*>(tasks + t) + 2);
+            const float tw[3] = {tk0.w, w12.x, w12.y};
+#pragma unroll
+            for (int c = 0; c < 3; ++c) lum[c] = sh.albedo[c] * (lum[c] * inv_ns) * tw[c];
+        }
+        *out = make_float4(lum[0], lum[1], lum[2], 0.f);
+    }
+    count_samples(n_shadow, ctr + 1);
 }
 
 // One warp per pixel. Its samples run side by side, G lanes each (G a power
@@ -897,20 +1021,20 @@ cudaError_t launch_render_count(const DevScene& sc, const DevCamera& cam, const 
     return cudaGetLastError();
 }
 
-// The k_shadow instance for (dtype, env, unit).
+// The k_shadow or k_shadow_env instance for (dtype, unit).
 template <int DT>
 static const void* shadow_kernel_dt(bool env, bool unit) {
-    if (env) return unit ? (const void*)k_shadow<DT, true, true> : (const void*)k_shadow<DT, true, false>;
-    return unit ? (const void*)k_shadow<DT, false, true> : (const void*)k_shadow<DT, false, false>;
+    if (env) return unit ? (const void*)k_shadow_env<DT, true> : (const void*)k_shadow_env<DT, false>;
+    return unit ? (const void*)k_shadow<DT, true> : (const void*)k_shadow<DT, false>;
 }
 static const void* shadow_kernel(int dtype, bool env, bool unit) {
     return dtype == 1 ? shadow_kernel_dt<1>(env, unit) : dtype == 2 ? shadow_kernel_dt<2>(env, unit)
                                                                     : shadow_kernel_dt<0>(env, unit);
 }
 
-// Resident CTAs per SM of the k_shadow instance for (dtype, env, unit), from
-// the occupancy calculator (once per instance; it enqueues no work, so it
-// may run while a stream is being captured).
+// Resident CTAs per SM of a shadow kernel instance, from the occupancy
+// calculator (once per instance; it enqueues no work, so it may run while a
+// stream is being captured).
 static int shadow_ctas_per_sm(int dtype, bool env, bool unit) {
     static std::atomic<int> cache[3][2][2];
     if (dtype < 0 || dtype > 2) dtype = 0;
@@ -921,6 +1045,40 @@ static int shadow_ctas_per_sm(int dtype, bool env, bool unit) {
         c.store((e == cudaSuccess && n > 0) ? n : 8);
     }
     return c.load();
+}
+
+// The shadow rays of environment light k.
+static cudaError_t launch_env_light(const DevScene& sc, int k, const ShadowTask* tasks, const int32_t* total,
+                                    int64_t task_cap, const RayOrder& ro, float4* direct, unsigned long long* counters,
+                                    int sms, cudaStream_t st) {
+    const bool unit = sc.smarch.unit != 0;
+    const unsigned blocks = (unsigned)sms * (unsigned)shadow_ctas_per_sm(sc.dens.dtype, true, unit);
+    const int ns = sc.lights[k].samples, per = ro.env.n_keys > 0 ? 1 : ns;
+    for (int s0 = 0; s0 < ns; s0 += per) {
+        cudaError_t e;
+        const int32_t* order = nullptr;
+        if (ro.env.n_keys > 0) {
+            if ((e = cudaMemsetAsync(ro.key_counts, 0, sizeof(int32_t) * ro.env.n_keys, st)) != cudaSuccess) return e;
+            k_env_keys<<<(unsigned)sms * 8u, 256, 0, st>>>(sc, ro.env, tasks, total, task_cap, k, s0, ro.key_counts);
+            ++g_launch_counter;
+            if ((e = launch_exclusive_scan(ro.key_counts, ro.env.n_keys, ro.key_offsets, ro.key_scan, ro.key_total,
+                                           st)) != cudaSuccess)
+                return e;
+            k_env_scatter<<<(unsigned)sms * 8u, 256, 0, st>>>(ro.env, total, task_cap, ro.key_offsets);
+            ++g_launch_counter;
+            order = ro.env.order;
+        }
+        unsigned long long* claim = counters + 5;
+        if ((e = cudaMemsetAsync(claim, 0, sizeof *claim, st)) != cudaSuccess) return e;
+        DevScene scv = sc;
+        int s1 = s0 + per;
+        void* args[] = {&scv, &k, &s0, &s1, &tasks, (void*)&total, &task_cap, &order, &direct, &counters, &claim};
+        if ((e = cudaLaunchKernel(shadow_kernel(sc.dens.dtype, true, unit), dim3(blocks), dim3(128), args, 0, st)) !=
+            cudaSuccess)
+            return e;
+        ++g_launch_counter;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_render_shade(const DevScene& sc, const DevCamera& cam, const DevScatterGrid& sg,
@@ -963,22 +1121,24 @@ cudaError_t launch_render_shade(const DevScene& sc, const DevCamera& cam, const 
             return e;
     }
     mark(1);
-    bool env = false;
-    for (int k = 0; k < sc.n_lights; ++k) env = env || sc.lights[k].type == 2;
     // one resident wave of CTAs; the threads stride over the rays
-    const bool unit = sc.smarch.unit != 0;
-    const unsigned sblocks = (unsigned)sms * (unsigned)shadow_ctas_per_sm(sc.dens.dtype, env, unit);
-    {
+    if (ro.rb.n > 0) {
+        const bool unit = sc.smarch.unit != 0;
+        const unsigned sblocks = (unsigned)sms * (unsigned)shadow_ctas_per_sm(sc.dens.dtype, false, unit);
         DevScene scv = sc;
         RayBins rbv = ro.rb;
         const ShadowTask* tasks_c = tasks;
         const int32_t* order_c = ro.order;
         void* args[] = {&scv, &rbv, &tasks_c, (void*)&total, &task_cap, &order_c, &direct, &counters};
-        if ((e = cudaLaunchKernel(shadow_kernel(sc.dens.dtype, env, unit), dim3(sblocks), dim3(128), args, 0, st)) !=
+        if ((e = cudaLaunchKernel(shadow_kernel(sc.dens.dtype, false, unit), dim3(sblocks), dim3(128), args, 0, st)) !=
             cudaSuccess)
             return e;
+        ++g_launch_counter;
     }
-    ++g_launch_counter;
+    for (int k = 0; k < sc.n_lights; ++k)
+        if (sc.lights[k].type == 2 &&
+            (e = launch_env_light(sc, k, tasks, total, task_cap, ro, direct, counters, sms, st)) != cudaSuccess)
+            return e;
     mark(2);
     k_resolve<<<(unsigned)((n_pix * 32 + 127) / 128), 128, 0, st>>>(cam, offsets, counts, pss, direct, sc.n_lights,
                                                                    task_cap, rgba, dfilm, sfilm, efilm);

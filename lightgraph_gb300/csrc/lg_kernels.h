@@ -171,7 +171,8 @@ size_t pixel_sample_bytes();
 //   kind 2 (environment light, random directions): task order in buckets of
 //          2^shift tasks.
 struct RayBin {
-    int kind, ns, nd, shift;  // ns: (u, v) or (s, t) bins per side (power of two), nd: depth bins
+    int kind, ns, nd;         // ns: (u, v) or (s, t) bins per side (power of two), nd: depth bins
+    int light;                // the scene's light
     float U[3], V[3], D[3];   // kind 0: orthonormal basis, D the ray direction
     float O[3];               // kind 1: light position (index space)
     float u0, v0, inv_bs;     // kind 0: projected origin, 1 / bin size
@@ -205,7 +206,7 @@ cudaError_t launch_expm1_check(const float* x, float* approx, float* ref, int n,
 // Initial value of a light's bound table entries (bits of a non-negative float).
 inline uint32_t bound_init(const RayBin& b) { return b.kind == 0 ? 0u : 0x7F800000u; }
 inline int64_t bound_entries(const RayBin& b) {
-    return b.kind == 0 ? (int64_t)b.ns * b.ns : b.kind == 1 ? 6 * (int64_t)b.ns * b.ns : 0;
+    return b.kind == 0 ? (int64_t)b.ns * b.ns : 6 * (int64_t)b.ns * b.ns;
 }
 // Wave 1: counts[ps] = shading samples of each pixel-sample.
 // claim: a zeroed counter the persistent grid's warps claim pixel samples
@@ -216,9 +217,21 @@ cudaError_t launch_render_count(const DevScene& sc, const DevCamera& cam, const 
 // Shadow-ray ordering buffers: key_counts and key_offsets hold rb's keys,
 // key_scan the scan's block sums (keys / 1024 + 2), order n_lights * units
 // (units of kRayUnit tasks).
+// Order of an environment light's shadow rays, a light sample at a time: by
+// direction (octahedral bins, 2^dir_bits a side), then by the start's cell
+// (2^cell_bits a side over the leaf bbox, Morton order). keys and order hold a
+// word per task.
+struct EnvOrder {
+    int dir_bits, cell_bits;
+    float lo[3], inv_cell;
+    uint32_t* keys;
+    int32_t* order;
+    int64_t n_keys;  // 0: the rays stay in task order
+};
 struct RayOrder {
     RayBins rb;
     int64_t n_keys;
+    EnvOrder env;
     int32_t *key_counts, *key_offsets, *key_scan, *key_total, *order;
     // the order key of every unit and light (light k's keys from
     // k * unit_cap), written by the primary shading pass with the counts
