@@ -252,10 +252,6 @@ cudaError_t launch_render_shade(const DevScene& sc, const DevCamera& cam, const 
 cudaError_t launch_exclusive_scan(const int32_t* in, int64_t n, int32_t* out, int32_t* block_sums, int32_t* total,
                                   cudaStream_t st);
 
-// Bounding box of the non-zero voxels of a dense array (array coordinates;
-// bbox pre-set to +/-INT_MAX).
-cudaError_t launch_voxel_bbox(const float* dense, const int dims[3], int* bbox, cudaStream_t st);
-
 // Dart throwing (LightGraph::scatterPoints), one CTA per iteration.
 struct DartParams {
     uint32_t scatter_count, target, batch, hard_limit;
@@ -287,13 +283,12 @@ cudaError_t launch_env_cdf(const float* rgb, int w, int h, float* cond_func, flo
                            int* cond_guide, int* marg_guide,
                            cudaStream_t st);
 
-// Grid upload helpers
-cudaError_t launch_pack_bricks(const float* dense, const int dims[3], const int origin[3],
-                               const DevGrid& g, void* bricks, cudaStream_t st);
-// bbox: 6 ints (min xyz, max xyz leaf coordinates), pre-set to +/-INT_MAX.
-cudaError_t launch_leaf_bits(const float* dense, const int dims[3], const int origin[3],
-                             const uint8_t* leaf_mask, const DevGrid& g, uint32_t* bits, int* bbox,
-                             cudaStream_t st);
+// Grid upload: the cell records, leaf and occupancy bitmaps (bitmap_words each,
+// cleared) and bounding boxes (12 ints, preset to +/-INT_MAX) of a dense array.
+inline size_t bitmap_words(const DevGrid& g) { return (size_t)g.nbits / 32 + 1; }
+cudaError_t launch_pack_volume(const float* dense, const int dims[3], const int origin[3], const uint8_t* leaf_mask,
+                               const DevGrid& g, void* bricks, uint32_t* leafbits, uint32_t* occbits, int* bbox,
+                               cudaStream_t st);
 
 extern std::atomic<uint64_t> g_launch_counter;  // kernel launches issued (all contexts, all host threads)
 // Raises a kernel's dynamic shared-memory limit on the current device, once

@@ -445,6 +445,7 @@ extern "C" lg_status lg_server_add_volume(lg_server* srv, const lg_grid_desc* de
         c.temp.valid = false;
         v->has_temp = true;
     }
+    c.staging.release();  // volumes come rarely here, and may be large
     std::lock_guard<std::mutex> lk2(srv->mu);
     srv->volumes.push_back(std::move(v));
     if (volume_id) *volume_id = (int32_t)srv->volumes.size() - 1;
