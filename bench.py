@@ -39,14 +39,17 @@ sys.path.insert(0, ROOT)
 
 STAGES = ["build_graph", "edge_march", "floyd_warshall", "vertex_light", "diffuse", "splat", "render"]
 NOMINAL_FP32_TFLOPS = 152 * 128 * 2 * 2.070 / 1000  # GB300: SMs x FP32 lanes x 2 (FMA) x 2.07 GHz
-FW_SCHEDULES = {0: "per-round launches", 1: "persistent 1 CTA/SM", 2: "persistent 2 CTA/SM",
+FW_SCHEDULES = {-1: "from the edges", 0: "per-round launches", 1: "persistent 1 CTA/SM", 2: "persistent 2 CTA/SM",
                 3: "symmetric persistent 1 CTA/SM", 4: "symmetric persistent 2 CTA/SM",
                 5: "symmetric persistent 2 CTA/SM, TMA-staged update operands"}
 def fw_executed_flops(ld, schedule):
     """FP32 ops (add + min per update) the solve's kernels execute for one
     ld x ld matrix: the general schedules run every (i, j, k); the symmetric
     ones the 128-tiles on and above the diagonal, the strip blocks and the
-    panel items of each of the nt = ld / 64 rounds."""
+    panel items of each of the nt = ld / 64 rounds. None for the solve from
+    the edges (-1), whose work depends on the graph."""
+    if schedule < 0:
+        return None
     if schedule < 3:
         return 2.0 * ld ** 3
     nt, nu = ld // 64, ld // 128
@@ -56,7 +59,7 @@ def fw_executed_flops(ld, schedule):
     return 2.0 * (tiles + strips + panels)
 
 
-FW_KERNELS = {0: "k_fw_update+k_fw_panels", 1: "k_fw_persistent", 2: "k_fw_persistent",
+FW_KERNELS = {-1: "k_path_prep+k_paths+k_path_mirror", 0: "k_fw_update+k_fw_panels", 1: "k_fw_persistent", 2: "k_fw_persistent",
               3: "k_fw_persistent_sym+k_fw_mirror", 4: "k_fw_persistent_sym+k_fw_mirror",
               5: "k_fw_persistent_sym<tma>+k_fw_mirror"}
 
@@ -192,8 +195,10 @@ def run_batched_graphs(local: int):
            "frame_ms_graph_replay": ev2.elapsed_time(ev3) / reps,
            "stages_ms": {k: round(float(v), 4) for k, v in zip(STAGES, stage)},
            "fw": {"schedule": FW_SCHEDULES.get(sched, str(sched)),
-                  "autotuner_ms": [round(x, 4) for x in tuned], "tflops": flops / (fw_ms * 1e-3) / 1e12,
-                  "frac_of_nominal_fp32": flops / (fw_ms * 1e-3) / 1e12 / NOMINAL_FP32_TFLOPS},
+                  "autotuner_ms": [round(x, 4) for x in tuned], "ms": fw_ms,
+                  "tflops": None if sched < 0 else flops / (fw_ms * 1e-3) / 1e12,
+                  "frac_of_nominal_fp32": None if sched < 0 else
+                  flops / (fw_ms * 1e-3) / 1e12 / NOMINAL_FP32_TFLOPS},
            "timing": "CUDA events on the frame stream, frames through lg_frame_device (graph build to render); "
                      "frame_ms with per-stage events, frame_ms_graph_replay as one captured CUDA graph"}
     ctx.close()
@@ -686,9 +691,10 @@ def run_ours(args):
     render_gbs = render_bytes / (stage_ms[6] * 1e-3) / 1e9
     ld = (len(pts) + 127) // 128 * 128  # the solve runs on the 128-padded matrix
     fw_sched, fw_tuned = ctx.fw_schedule()
-    fw_flops = 2.0 * ld ** 3
-    fw_tflops = fw_flops / (stage_ms[2] * 1e-3) / 1e12
+    # rates count the dense solve's operations: none for a solve from the edges
     fw_exec = fw_executed_flops(ld, fw_sched)
+    fw_tflops = fw_exec and 2.0 * ld ** 3 / (stage_ms[2] * 1e-3) / 1e12
+    fw_exec_tflops = fw_exec and fw_exec / (stage_ms[2] * 1e-3) / 1e12
     fw_ceiling = ctx.fw_inner_loop_rate()
     line = {
         "metric": "ms/frame", "value": value, "unit": "ms", "n_gpus": world, "steps": args.steps,
@@ -710,15 +716,16 @@ def run_ours(args):
         "render_stage": {"ms": float(stage_ms[6]), "algorithmic_bytes": render_bytes, "achieved_gbs": render_gbs,
                          "frac": render_gbs / peaks.get("hbm_gbs")},
         "fw_roofline": {"kernel": FW_KERNELS.get(fw_sched, "?"),
-                        "bound": "fp32_alu", "n": int(ld),
+                        "bound": "fp32_alu" if fw_exec else "shared memory", "n": int(ld),
+                        "launch_ms": float(stage_ms[2]),
                         "achieved": fw_tflops, "unit": "TFLOP/s", "peak": NOMINAL_FP32_TFLOPS,
                         "peak_kind": "nominal (152 SMs x 128 lanes x 2 x 2.07 GHz)",
-                        "frac": fw_tflops / NOMINAL_FP32_TFLOPS,
+                        "frac": fw_tflops and fw_tflops / NOMINAL_FP32_TFLOPS,
                         "schedule": FW_SCHEDULES.get(fw_sched, str(fw_sched)),
                         "autotuner_ms": [round(x, 4) for x in fw_tuned],
-                        "executed_tflops": fw_exec / (stage_ms[2] * 1e-3) / 1e12,
+                        "executed_tflops": fw_exec_tflops,
                         "inner_loop_ceiling_tflops": fw_ceiling,
-                        "executed_frac_of_inner_loop_ceiling": fw_exec / (stage_ms[2] * 1e-3) / 1e12 / fw_ceiling},
+                        "executed_frac_of_inner_loop_ceiling": fw_exec_tflops and fw_exec_tflops / fw_ceiling},
     }
     if rank == 0 and args.serving > 0:
         line["serving"] = run_serving(args.serving, [float(r) for r in args.rates.split(",") if r])

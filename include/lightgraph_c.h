@@ -362,20 +362,25 @@ lg_status lg_set_graph_mode(lg_ctx* ctx, int on);
 /* Kernels in one captured frame (0 before the first capture). */
 uint64_t lg_frame_launches(const lg_ctx* ctx);
 
-/* Schedule of the path solve over all loaded graphs. -1 (default): chosen by
- * the autotuner, which times every candidate once per (graph count, largest
- * graph) on a scratch copy and keeps the fastest; 0: two launches per round
+/* Schedule of the path solve over all loaded graphs. -1 (default): a single
+ * graph, or several of which one has more than 2048 points, is solved from its
+ * edges (up to 9200 points a graph and 16 edges a point; distances are sums
+ * along a shortest path rounded to FP32 once, with infinity where the squared
+ * transmittance underflows in FP64); others by Floyd-Warshall on the schedule
+ * chosen by the autotuner, which times every candidate once per (graph count,
+ * largest graph) on a scratch copy and keeps the fastest; 0: two launches per round
  * per graph; 1 or 2: one persistent launch for every graph with 1 or 2 CTAs
  * per SM (a work queue with per-graph dependency counters); 3 or 4: the
  * symmetric persistent solve (for the symmetric matrices the graph stage
  * builds) with 1 or 2 CTAs per SM; 5: schedule 4 with the update tiles'
  * operands staged into shared memory by TMA bulk copies (cp.async.bulk on an
- * mbarrier) instead of through registers. All schedules give the same
+ * mbarrier) instead of through registers. Schedules 0 to 5 give the same
  * distances bit for bit. A schedule set here stays in force for later graph
  * builds until -1 is set again. */
 lg_status lg_set_fw_schedule(lg_ctx* ctx, int schedule);
-/* The schedule in use and the autotuner's timings (ms) of schedules 0..5
- * (0 for a schedule it did not time).
+/* The schedule in use (-1: none chosen, as while graphs are solved from their
+ * edges) and the autotuner's timings (ms) of schedules 0..5 (0 for a schedule
+ * it did not time).
  * Returns LG_ERR_TIMEOUT if a persistent solve reported a stalled queue. */
 lg_status lg_fw_schedule(lg_ctx* ctx, int* schedule, double* tuned_ms, int n);
 /* The ceiling of the Floyd-Warshall update tiles on this GPU: FP32 ops/s

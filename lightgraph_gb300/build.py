@@ -36,7 +36,7 @@ LIB_NAME = "liblightgraph_gb300.so"
 HOST_LIB_NAME = "liblightgraph_host.so"
 ORACLE_NAME = "liblg_oracle.so"
 
-CU_SOURCES = ["lg_api.cu", "k_graph.cu", "k_march.cu", "k_fw.cu", "k_diffuse.cu", "k_splat.cu",
+CU_SOURCES = ["lg_api.cu", "k_graph.cu", "k_march.cu", "k_fw.cu", "k_paths.cu", "k_diffuse.cu", "k_splat.cu",
               "k_render.cu", "k_grid.cu", "k_dart.cu", "lg_server.cu", "lg_noalloc.cu"]
 HOST_SOURCES = ["scene.cc", "lg_parse.cc", "lg_exr.cc"]
 CLI_SOURCE = "cli.cc"

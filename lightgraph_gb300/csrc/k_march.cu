@@ -16,7 +16,7 @@ __global__ void __launch_bounds__(128) k_edge_march(DevScene sc, const float* __
                                                     const GraphInfo* __restrict__ graphs,
                                                     const int2* __restrict__ edges,
                                                     const int32_t* __restrict__ edge_cnt,
-                                                    float* __restrict__ S) {
+                                                    float* __restrict__ S, float* __restrict__ W) {
     const GraphInfo g = graphs[blockIdx.y];
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= edge_cnt[blockIdx.y]) return;
@@ -50,6 +50,10 @@ __global__ void __launch_bounds__(128) k_edge_march(DevScene sc, const float* __
         if (march_fixed<DT>(G, r, sc.step1, scale, sh.dMax, sh.tau_drop, contrib, tau, dropped, ns)) {
             value = dropped ? kInf : tau;
         }
+    }
+    if (W) {  // one depth per edge, for the solve from the edges
+        W[g.e_off + e] = value;
+        return;
     }
     float* M = S + g.s_off;
     M[(int64_t)ij.x * g.ld + ij.y] = value;
@@ -170,12 +174,12 @@ __global__ void __launch_bounds__(128) k_vertex_light(DevScene sc, const float* 
 
 cudaError_t launch_edge_march(const DevScene& sc, const float* pts, const GraphInfo* graphs,
                               int n_graphs, int max_edges, const int2* edges,
-                              const int32_t* edge_cnt, float* S, cudaStream_t st) {
+                              const int32_t* edge_cnt, float* S, float* W, cudaStream_t st) {
     if (n_graphs == 0 || max_edges == 0) return cudaSuccess;
     dim3 grid((max_edges + 127) / 128, n_graphs);
-    if (sc.dens.dtype == 1) k_edge_march<1><<<grid, 128, 0, st>>>(sc, pts, graphs, edges, edge_cnt, S);
-    else if (sc.dens.dtype == 2) k_edge_march<2><<<grid, 128, 0, st>>>(sc, pts, graphs, edges, edge_cnt, S);
-    else k_edge_march<0><<<grid, 128, 0, st>>>(sc, pts, graphs, edges, edge_cnt, S);
+    if (sc.dens.dtype == 1) k_edge_march<1><<<grid, 128, 0, st>>>(sc, pts, graphs, edges, edge_cnt, S, W);
+    else if (sc.dens.dtype == 2) k_edge_march<2><<<grid, 128, 0, st>>>(sc, pts, graphs, edges, edge_cnt, S, W);
+    else k_edge_march<0><<<grid, 128, 0, st>>>(sc, pts, graphs, edges, edge_cnt, S, W);
     ++g_launch_counter;
     return cudaGetLastError();
 }

@@ -689,6 +689,7 @@ lg_status Ctx::load_graphs(int n_graphs, const float* points, const int64_t* off
         for (auto& kv : fw_tuned)
             if (kv.first == std::make_pair(n_graphs, max_n)) fw_choice = kv.second;
     graphs_built = false;
+    marched.valid = false;
     return LG_OK;
 }
 
@@ -943,7 +944,73 @@ lg_status Ctx::march_edges() {
     CK(d_S.reserve(sizeof(float) * std::max<int64_t>(s_floats, 1)), "S alloc");
     CK(launch_fill(d_S.as<float>(), s_floats, INFINITY, st), "S fill");
     CK(launch_edge_march(scene(), d_pts.as<float>(), d_graphs.as<GraphInfo>(), n_graphs, max_edges,
-                         d_edges.as<int2>(), d_edge_cnt.as<int32_t>(), d_S.as<float>(), st), "edge march");
+                         d_edges.as<int2>(), d_edge_cnt.as<int32_t>(), d_S.as<float>(), nullptr, st), "edge march");
+    marched = {true, {shader.extinction[0], shader.extinction[1], shader.extinction[2], settings.cutoff}};
+    return LG_OK;
+}
+
+bool Ctx::marched_as_set() const {
+    return marched.valid && marched.by[0] == shader.extinction[0] && marched.by[1] == shader.extinction[1] &&
+           marched.by[2] == shader.extinction[2] && marched.by[3] == settings.cutoff;
+}
+
+// Whether the paths are solved from the edges (k_paths.cu), and in which unit: as
+// fine as lets 32 bits hold a depth R at which the squared transmittance of
+// every channel underflows in FP64 (2 a R > 745), where the reference's
+// comparison of squared lengths sees no path, plus one edge.
+// Floyd-Warshall solves the graphs where a schedule is pinned, a graph is too
+// large for shared memory or has too many edges, depths could be negative (only
+// a negative cutoff lets them through), a channel does not absorb, and in
+// batches of graphs of up to 2048 points, where it fills the GPU and is as fast
+// or faster (16 of 500 points: 0.24 against 0.31 ms, 8 of 1025: 0.70 against
+// 0.67 ms, 4 of 1500: 0.77 against 0.91 ms; 2 of 2100: 1.00 against 0.87 ms).
+bool Ctx::path_unit(PathUnit& pu) const {
+    if (fw_pinned >= 0 || settings.cutoff < 0.0 || max_n > kPathMaxPoints || max_connect > 16) return false;
+    if (n_graphs > 1 && max_n <= 2048) return false;
+    double a[3], lo = INFINITY, hi = 0.0;
+    for (int c = 0; c < 3; ++c) {
+        a[c] = -shader.extinction[c];
+        lo = std::min(lo, a[c]);
+        hi = std::max(hi, a[c]);
+    }
+    if (!(lo > 1e-30) || !(hi < 1e30) || hi > 4.0 * lo) return false;
+    const double R = 373.0 / lo;
+    // an edge that did not drop out is no deeper than the dropout depth
+    const double edge = std::min(R, 1.0001 * (double)std::max(dropout_depth(a, settings.cutoff), 0.f));
+    if (!(edge > 0.0)) return false;  // every edge drops out
+    pu.per_unit = 4294960000.0 / (R + edge);
+    pu.longest = (float)edge;
+    pu.far = (uint32_t)(R * pu.per_unit);
+    return true;
+}
+
+lg_status Ctx::march_to_edges() {
+    Ctx* ctx = this;
+    if (!D().valid) return fail(LG_ERR_STATE, "no density grid uploaded");
+    if (!graphs_built) return fail(LG_ERR_STATE, "no graphs built");
+    CK(d_S.reserve(sizeof(float) * std::max<int64_t>(s_floats, 1)), "S alloc");
+    CK(d_edge_depth.reserve(sizeof(float) * std::max<int64_t>(edge_slots, 1)), "edge depth alloc");
+    CK(launch_edge_march(scene(), d_pts.as<float>(), d_graphs.as<GraphInfo>(), n_graphs, max_edges,
+                         d_edges.as<int2>(), d_edge_cnt.as<int32_t>(), nullptr, d_edge_depth.as<float>(), st),
+       "edge march");
+    return LG_OK;
+}
+
+lg_status Ctx::solve_from_edges(const PathUnit& pu) {
+    Ctx* ctx = this;
+    marched.valid = false;
+    const int64_t P = std::max<int64_t>(n_points, 1);
+    CK(d_path_order.reserve(2 * sizeof(uint16_t) * P), "path order alloc");
+    const size_t places = (size_t)P * path_stride(max_connect);
+    CK(d_path_ell.reserve((sizeof(int2) + sizeof(uint32_t)) * places), "path edges alloc");
+    CK(d_path_step.reserve(sizeof(uint32_t) * n_graphs), "path step alloc");
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "device query");
+    const PathScratch ps = {d_path_order.as<uint16_t>(), d_path_order.as<uint16_t>() + P, d_path_ell.as<int4>(),
+                            reinterpret_cast<uint32_t*>(d_path_ell.as<int2>() + places), d_path_step.as<uint32_t>()};
+    CK(launch_paths(d_pts.as<float>(), d_graphs.as<GraphInfo>(), n_graphs, max_n, n_points, max_connect,
+                    d_edges.as<int2>(), d_edge_cnt.as<int32_t>(), d_edge_depth.as<float>(), pu, ps, d_S.as<float>(),
+                    sms, st), "paths from the edges");
     return LG_OK;
 }
 
@@ -1135,6 +1202,15 @@ lg_status Ctx::tune_fw() {
 
 lg_status Ctx::solve_paths() {
     Ctx* ctx = this;
+    PathUnit pu;
+    const bool from_edges = marched_as_set() && path_unit(pu);
+    marched.valid = false;
+    if (from_edges) {
+        CK(d_edge_depth.reserve(sizeof(float) * std::max<int64_t>(edge_slots, 1)), "edge depth alloc");
+        CK(launch_edge_depths(d_graphs.as<GraphInfo>(), n_graphs, max_edges, d_edges.as<int2>(),
+                              d_edge_cnt.as<int32_t>(), d_S.as<float>(), d_edge_depth.as<float>(), st), "edge depths");
+        return solve_from_edges(pu);
+    }
     if (fw_choice < 0) {
         lg_status s = tune_fw();
         if (s != LG_OK) return s;
@@ -1243,9 +1319,11 @@ extern "C" lg_status lg_diffuse(lg_ctx* handle, float* diffuse_out) {
 }
 
 lg_status Ctx::solve_all() {
-    lg_status s = march_edges();
+    PathUnit pu;
+    const bool from_edges = path_unit(pu);
+    lg_status s = from_edges ? march_to_edges() : march_edges();
     if (s != LG_OK) return s;
-    s = solve_paths();
+    s = from_edges ? solve_from_edges(pu) : solve_paths();
     if (s != LG_OK) return s;
     paths_solved = true;
     s = vertex_light();
@@ -1882,9 +1960,14 @@ lg_status Ctx::frame_enqueue(double point_voxel_size, const lg_camera* camera) {
     lg_status s = render_count_early(camera);
     if (s == LG_OK) s = build_edges();
     mark(1);
-    if (s == LG_OK) s = march_edges();
+    PathUnit pu;
+    const bool from_edges = path_unit(pu);
+    if (s == LG_OK) s = from_edges ? march_to_edges() : march_edges();
     mark(2);
-    if (s == LG_OK) { s = solve_paths(); paths_solved = s == LG_OK; }
+    if (s == LG_OK) {
+        s = from_edges ? solve_from_edges(pu) : solve_paths();
+        paths_solved = s == LG_OK;
+    }
     mark(3);
     if (s == LG_OK) { s = vertex_light(); light_done = s == LG_OK; }
     mark(4);

@@ -97,6 +97,8 @@ struct Ctx {
     bool graphs_built = false, paths_solved = false, light_done = false, diffuse_done = false;
     DevBuf d_pts, d_graphs, d_pt_graph, d_cand, d_cand_cnt, d_pairs, d_edges, d_edge_cnt, d_adj, d_adj_off;
     DevBuf d_S, d_L, d_D, d_part, d_colw, d_fw;
+    // the solve from the edges: depth per edge, vertex order, edge places
+    DevBuf d_edge_depth, d_path_order, d_path_ell, d_path_step;
 
     // batched Floyd-Warshall: work queue, counters and the autotuned schedule
     DevBuf d_fwg, d_fw_items, d_fw_sync, d_fw_tune;
@@ -196,6 +198,19 @@ struct Ctx {
     std::vector<int32_t> h_dart_cnt;
     lg_status march_edges();
     lg_status solve_paths();
+    // The solve from the edges (k_paths.cu), where path_unit says so, instead
+    // of Floyd-Warshall; march_to_edges is march_edges without the matrix, for
+    // the calls between whose stages nobody sees it
+    bool path_unit(PathUnit& pu) const;
+    // What march_edges left in the matrices: depths cut off for this extinction
+    // and cutoff, until a solve or another set of graphs takes their place
+    struct Marched {
+        bool valid = false;
+        double by[4] = {0.0, 0.0, 0.0, 0.0};
+    } marched;
+    bool marched_as_set() const;
+    lg_status march_to_edges();
+    lg_status solve_from_edges(const PathUnit& pu);
     lg_status vertex_light();
     lg_status diffuse();
     lg_status solve_all();

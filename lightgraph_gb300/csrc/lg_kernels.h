@@ -48,11 +48,40 @@ cudaError_t launch_adjacency(const GraphInfo* graphs, int n_graphs, int max_edge
                              const int64_t* adj_off, cudaStream_t st);
 cudaError_t launch_fill(float* p, int64_t n, float v, cudaStream_t st);
 
+// W == nullptr: both entries of each edge in the matrices S; else one depth per
+// edge slot in W.
 cudaError_t launch_edge_march(const DevScene& sc, const float* pts, const GraphInfo* graphs,
                               int n_graphs, int max_edges, const int2* edges,
-                              const int32_t* edge_cnt, float* S, cudaStream_t st);
+                              const int32_t* edge_cnt, float* S, float* W, cudaStream_t st);
 cudaError_t launch_vertex_light(const DevScene& sc, const float* pts, const GraphInfo* graphs,
                                 int n_graphs, int max_n, float* L, cudaStream_t st);
+
+// All-pairs paths of the graphs from their edges' depths W into the matrices S
+// (distances, diagonal 0, padding inf). Scratch: perm and rank a half-word per
+// point, ell path_stride / 2 places and rest path_stride words a point, step a
+// word per graph.
+// Distances are counted in units: `far` of them and more are no path, and an
+// edge no longer than `longest` added to far still fits 32 bits.
+struct PathUnit {
+    double per_unit;
+    float longest;
+    uint32_t far;
+};
+struct PathScratch {
+    uint16_t *perm, *rank;
+    int4* ell;
+    uint32_t* rest;
+    uint32_t* step;
+};
+constexpr int kPathMaxPoints = 9200;  // K = 4 distances of a graph in shared memory
+int path_stride(int max_connect);
+cudaError_t launch_paths(const float* pts, const GraphInfo* graphs, int n_graphs, int max_n, int64_t n_points,
+                         int max_connect, const int2* edges, const int32_t* edge_cnt, const float* W, const PathUnit& pu,
+                         const PathScratch& ps, float* S, int sms, cudaStream_t st);
+
+// The edges' depths W from the matrices S.
+cudaError_t launch_edge_depths(const GraphInfo* graphs, int n_graphs, int max_edges, const int2* edges,
+                               const int32_t* edge_cnt, const float* S, float* W, cudaStream_t st);
 
 // Floyd-Warshall on one matrix (general, any n, ld % 4 == 0).
 cudaError_t fw_solve(float* d, int n, int ld, cudaStream_t st);

@@ -281,7 +281,7 @@ void lg_server::run(Slot* s, Request* q) {
     // residency, so the slots' solves may share the SMs; measured 11% more
     // renders/s than 1 CTA per SM on the mixed stream), its queue in
     // structural order (one-off sizes do not pay for the list scheduling)
-    if (st == LG_OK) c.fw_choice = 4;
+    if (st == LG_OK) c.fw_pinned = c.fw_choice = 4;
     if (st == LG_OK) st = c.build_edges();
     if (opts.solo_paths) {
         if (st == LG_OK) st = c.solve_all();
