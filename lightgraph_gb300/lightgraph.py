@@ -13,6 +13,9 @@ the calls raise.
 from __future__ import annotations
 
 import ctypes as C
+import math
+import sys
+import threading
 from dataclasses import dataclass, field
 from typing import Sequence
 
@@ -233,6 +236,45 @@ class Films:
 # device context
 # ---------------------------------------------------------------------------
 
+def _references(blocks: list, k: int) -> int:
+    return sys.getrefcount(blocks[k])
+
+
+_UNSHARED = _references([np.empty(1)], 0)
+
+
+class _ResultBlocks:
+    """Host memory of large results, used again once the caller has dropped every
+    array on it. Fresh pages cost more than the download that fills them: 64 MB
+    of films take 0.4 ms into pages in use and 1.6 ms into new ones, and whether
+    the C library's heap hands out new ones varies from process to process (a
+    256 x 256 frame took 1.4 or 2.3 ms). Results are views; a block that only
+    the pool refers to is free. Knows the last KEEP blocks of at least SMALLEST
+    bytes (below, a view costs as much as it saves), together at most LIMIT."""
+
+    KEEP, LIMIT, SMALLEST = 8, 256 << 20, 256 << 10
+
+    def __init__(self):
+        self.blocks: list[np.ndarray] = []  # least recently used first
+        self.lock = threading.RLock()
+
+    def empty(self, shape) -> np.ndarray:
+        """An FP32 array of this shape with any contents."""
+        n = math.prod(shape)
+        if 4 * n < self.SMALLEST:
+            return np.empty(shape, np.float32)
+        with self.lock:
+            for k in range(len(self.blocks)):
+                if self.blocks[k].size == n and _references(self.blocks, k) == _UNSHARED:
+                    self.blocks.append(self.blocks.pop(k))
+                    return self.blocks[-1].reshape(shape)
+            self.blocks.append(np.empty(n, np.float32))
+            out = self.blocks[-1].reshape(shape)
+            while len(self.blocks) > self.KEEP or sum(b.nbytes for b in self.blocks) > self.LIMIT:
+                self.blocks.pop(0)
+            return out
+
+
 class Context:
     """One CUDA device and stream with the resident grids and stage buffers."""
 
@@ -245,6 +287,7 @@ class Context:
         self.h = h
         self._graph_sizes: list[int] = []
         self._film_shape = (0, 0)
+        self._results = _ResultBlocks()
 
     def close(self) -> None:
         if self.h:
@@ -369,7 +412,7 @@ class Context:
         dims = (C.c_int32 * 3)()
         lo = (C.c_int32 * 3)()
         self._ck(self.lib.lg_get_scatter_grid(self.h, dims, lo, None))
-        vals = np.empty((dims[2], dims[1], dims[0], 3), np.float32)
+        vals = self._results.empty((dims[2], dims[1], dims[0], 3))
         self._ck(self.lib.lg_get_scatter_grid(self.h, dims, lo, ptr(vals)))
         return tuple(lo), tuple(dims), vals
 
@@ -377,7 +420,7 @@ class Context:
     def render(self, opts: SceneSettings) -> Films:
         cam = opts.camera_c()
         shape = (opts.height, opts.width, 4)
-        films = [np.empty(shape, np.float32) for _ in range(4)]
+        films = [self._results.empty(shape) for _ in range(4)]
         self._ck(self.lib.lg_render(self.h, C.byref(cam), *[ptr(f) for f in films]))
         return Films(*films)
 
@@ -407,7 +450,7 @@ class Context:
         r2 = np.asarray(radius_sq, dtype=np.float32)
         cam = opts.camera_c()
         shape = (opts.height, opts.width, 4)
-        films = [np.empty(shape, np.float32) for _ in range(4)]
+        films = [self._results.empty(shape) for _ in range(4)]
         self._ck(self.lib.lg_render_frame(self.h, len(points), ptr(pts), ptr(offs), ptr(r2), max_connect,
                                           point_voxel_size, C.byref(cam), *[ptr(f) for f in films]))
         self._graph_sizes = [len(p) for p in points]
@@ -448,12 +491,14 @@ class Context:
     def films(self, opts: SceneSettings) -> Films:
         """The films of the last render or frame_device (waits for it)."""
         shape = (opts.height, opts.width, 4)
-        films = [np.empty(shape, np.float32) for _ in range(4)]
+        films = [self._results.empty(shape) for _ in range(4)]
         self._ck(self.lib.lg_get_films(self.h, *[ptr(f) for f in films]))
         return Films(*films)
 
     def fw_host(self, S: np.ndarray) -> np.ndarray:
-        out = np.ascontiguousarray(S, dtype=np.float32).copy()
+        S = np.ascontiguousarray(S, dtype=np.float32)
+        out = self._results.empty(S.shape)
+        out[...] = S
         self._ck(self.lib.lg_fw_host(self.h, ptr(out), out.shape[0]))
         return out
 
