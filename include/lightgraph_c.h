@@ -363,14 +363,15 @@ lg_status lg_set_graph_mode(lg_ctx* ctx, int on);
 uint64_t lg_frame_launches(const lg_ctx* ctx);
 
 /* Schedule of the path solve over all loaded graphs. -1 (default): a single
- * graph, or several of which one has more than 2048 points, is solved from its
- * edges (up to 9200 points a graph and 16 edges a point; distances are sums
- * along a shortest path rounded to FP32 once, with infinity where the squared
- * transmittance underflows in FP64); others by Floyd-Warshall on the schedule
- * chosen by the autotuner, which times every candidate once per (graph count,
- * largest graph) on a scratch copy and keeps the fastest; 0: two launches per round
- * per graph; 1 or 2: one persistent launch for every graph with 1 or 2 CTAs
- * per SM (a work queue with per-graph dependency counters); 3 or 4: the
+ * graph, a few small ones (up to eight of together 4096 points) and batches with
+ * large ones are solved from their edges, up to 9200 points a graph and 16 edges
+ * a point (a distance is the sum along a shortest path, rounded to FP32 once,
+ * and infinity where its squared transmittance underflows in FP64); others by
+ * Floyd-Warshall on the schedule chosen by the autotuner, which times every
+ * candidate once per (graph count, largest graph) on a scratch copy and keeps
+ * the fastest; 0: two launches per round per graph; 1 or 2: one persistent
+ * launch for every graph with 1 or 2 CTAs per SM (a work queue with per-graph
+ * dependency counters); 3 or 4: the
  * symmetric persistent solve (for the symmetric matrices the graph stage
  * builds) with 1 or 2 CTAs per SM; 5: schedule 4 with the update tiles'
  * operands staged into shared memory by TMA bulk copies (cp.async.bulk on an

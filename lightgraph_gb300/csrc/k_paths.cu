@@ -284,7 +284,8 @@ __global__ void __launch_bounds__(1024) k_paths(const GraphInfo* __restrict__ gr
     }
     __syncthreads();
     if (tid < ns) reinterpret_cast<uint32_t*>(d)[(s0 + tid) * K + tid] = 0u;
-    uint32_t bound = step;
+    uint32_t bound = min(step, far - 1u);
+    const bool small = n <= 4 * nt;
     for (int par = 0;; par ^= 1) {
         // 1. the vertices whose distances fell to the bound or below, and the
         // least of the others'
@@ -367,7 +368,13 @@ __global__ void __launch_bounds__(1024) k_paths(const GraphInfo* __restrict__ gr
                 atomicMin(pending + v, f);
             }
         }
-        bound = items > 0 ? min(bound, far - step) + step : waiting;
+        // In a small graph the bound grows faster where a pass leaves threads idle
+        // (200 points: 0.070 -> 0.055 ms, of them chains of few neighbours 0.19 ->
+        // 0.07 ms; 4096 points: 2.23 -> 2.36 ms, so not in a large one). It stays
+        // below far, the mark of vertices with nothing pending.
+        const uint32_t by = small && items > 0 ? (uint32_t)min(max(nt / items, 1), 4) : 1u;
+        const uint32_t room = far - 1u - bound;
+        bound = items == 0 ? waiting : room / by > step ? bound + by * step : far - 1u;
         __syncthreads();
     }
     // The edge by which each distance came: of those that give it, the one to

@@ -496,9 +496,7 @@ class Context:
         return Films(*films)
 
     def fw_host(self, S: np.ndarray) -> np.ndarray:
-        S = np.ascontiguousarray(S, dtype=np.float32)
-        out = self._results.empty(S.shape)
-        out[...] = S
+        out = np.ascontiguousarray(S, dtype=np.float32).copy()
         self._ck(self.lib.lg_fw_host(self.h, ptr(out), out.shape[0]))
         return out
 

@@ -1,5 +1,5 @@
 """The path solve from the edges (k_paths.cu), which runs where no Floyd-Warshall
-schedule is pinned: graph sizes around a source group, a mark
+schedule is pinned and the graphs are few or large: graph sizes around a source group, a mark
 word and the sizes at which the group or the thread count changes, edge caps
 off the usual 12, graphs in several pieces and empty ones, batches of mixed
 sizes. The diffused radiances against the oracle's (FP64 Dijkstra over the
@@ -62,7 +62,7 @@ def test_sizes(gpu_ctx, scene, cap):
     solve(gpu_ctx, scene, clouds + [cloud(scene, 2049, 3)], [0.12] * (len(sizes) + 1), cap)
 
 
-@pytest.mark.parametrize("sizes", [[1700, 1701, 2049, 300], [3040, 3041, 17], [1672], [1673], [2432], [2433], [700] * 5])
+@pytest.mark.parametrize("sizes", [[1700, 1701, 2049, 300], [3040, 3041, 17], [1672], [1673], [2432], [2433], [700] * 5, [512] * 8, [300] * 9, [2300] + [400] * 16, [2300] + [900] * 16, [820] * 5])
 def test_group_sizes(gpu_ctx, scene, sizes):
     clouds = [cloud(scene, n, 7 + k) for k, n in enumerate(sizes)]
     solve(gpu_ctx, scene, clouds, [float(1.3 * n ** (-1.0 / 3.0)) for n in sizes], 12)
