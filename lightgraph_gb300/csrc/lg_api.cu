@@ -823,6 +823,8 @@ lg_status Ctx::scatter_points(const lg_scatter_opts& o, int first_iter, int n_it
     CK(cudaMemcpyAsync(h_dart_m2.data(), d_dart_m2.p, sizeof(float) * n_iter, cudaMemcpyDeviceToHost, st),
        "dart download");
     CK(cudaStreamSynchronize(st), "dart sync");
+    for (int32_t c : h_dart_cnt)
+        if (c < 0) return fail(LG_ERR_TIMEOUT, "dart throwing: a wait between CTAs ran out");
     return LG_OK;
 }
 

@@ -91,3 +91,27 @@ def test_scatter_points_chunk_edges(gpu_ctx, kw, dtype, origin):
         assert np.array_equal(pts[i].view(np.uint32), opt[i, :ocnt[i]].view(np.uint32))
         # (an expected size of 0 makes the radius NaN, on both sides)
         assert np.array_equal(np.float32(r2[i]), connect_r2(om2[i], opts.connect_mult), equal_nan=True)
+
+
+@pytest.mark.parametrize("kw", [
+    dict(scatter_count=3327, n_estimates=4),                 # below one chunk of 3328 candidates
+    dict(scatter_count=3 * 3328 + 1, n_estimates=1),         # as many chunks as slots, and one candidate
+    dict(scatter_count=7 * 3328, n_estimates=7),             # a radius update at the end of every chunk
+    dict(scatter_count=30000, n_estimates=18, target_size=5, hard_limit=7),  # ends early, helpers ahead
+    dict(scatter_count=30000, target_size=4000, hard_limit=4096, min_dist_mult=0.01),
+])
+def test_scatter_points_batch_sizes(gpu_ctx, kw):
+    """A cluster of three CTAs an iteration, of two, one CTA alone, and two to
+    an SM, by the number of iterations: the same points bit for bit, the first
+    and last the oracle's."""
+    sc = scenes.small(n_points=16, res=64)
+    scenes.load_into(gpu_ctx, sc)
+    opts = lgm.scatter_opts(**kw)
+    pts, r2 = gpu_ctx.scatter_points(3, 170, opts)
+    for n in (1, 24, 45, 60, 76, 100):
+        p, q = gpu_ctx.scatter_points(3, n, opts)
+        assert np.array_equal(np.asarray(q), np.asarray(r2)[:n], equal_nan=True)
+        for i in range(n):
+            assert np.array_equal(p[i].view(np.uint32), pts[i].view(np.uint32)), (n, i)
+    check_iterations(gpu_ctx, sc, opts, 3, 1)
+    check_iterations(gpu_ctx, sc, opts, 172, 1)
