@@ -264,6 +264,7 @@ __device__ __forceinline__ void mt_next_chunk(const uint32_t* cur, uint32_t* nxt
             if (third) out[t + 454] = mt_twist_word(a2, b2, x);
         }
         prev = out;
+        __syncwarp();  // a warp has to arrive as a whole
         asm volatile("bar.sync 1, %0;" ::"n"(kDartTwisters) : "memory");
     }
 }

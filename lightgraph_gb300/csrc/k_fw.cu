@@ -224,9 +224,8 @@ __device__ __forceinline__ void panel_product(const PanelSmem& sm, bool row_pane
 // it is already closed in d (the persistent schedule closes it once, in its
 // own item).
 template <bool kL2>
-__device__ __forceinline__ void fw_panel_tile(float* __restrict__ d, int n, int ld, int kb, int b, PanelSmem& sm,
+__device__ __forceinline__ void fw_panel_tile(float* __restrict__ d, int n, int ld, int nt, int kb, int b, PanelSmem& sm,
                                               bool closed_diag = false) {
-    const int nt = (n + kKB - 1) / kKB;
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
     const int K0 = kb * kKB;
     int kind = 0, other = kb;  // 0 diag, 1 row tile (K0, other), 2 col tile (other, K0)
@@ -237,11 +236,34 @@ __device__ __forceinline__ void fw_panel_tile(float* __restrict__ d, int n, int 
         other = q < kb ? q : q + 1;
     }
     const int O0 = other * kKB;
-    for (int e = tid; e < kKB * kKB; e += 256) {
-        const int r = e >> 6, c = e & 63;
-        sm.Dg[r][c] = ld_or_inf<kL2>(d, n, ld, K0 + r, K0 + c);
-        if (kind != 0)
-            sm.T[r][c] = kind == 1 ? ld_or_inf<kL2>(d, n, ld, K0 + r, O0 + c) : ld_or_inf<kL2>(d, n, ld, O0 + r, K0 + c);
+    // 16 bytes a load: 11 us a launch of k_fw_panels at n = 1021, 17.6 with 4 bytes
+    const int R0 = kind == 2 ? O0 : K0, C0 = kind == 2 ? K0 : O0;  // the panel tile's corner
+    if (max(K0, O0) + kKB <= n) {
+        float4 dg[4], pt[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int r = (tid >> 4) + 16 * q, c = (tid & 15) * 4;
+            dg[q] = ldm4<kL2>(d + (int64_t)(K0 + r) * ld + K0 + c);
+            if (kind != 0) pt[q] = ldm4<kL2>(d + (int64_t)(R0 + r) * ld + C0 + c);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int r = (tid >> 4) + 16 * q, c = (tid & 15) * 4;
+            float2* to = reinterpret_cast<float2*>(&sm.Dg[r][c]);
+            to[0] = make_float2(dg[q].x, dg[q].y);
+            to[1] = make_float2(dg[q].z, dg[q].w);
+            if (kind != 0) {
+                to = reinterpret_cast<float2*>(&sm.T[r][c]);
+                to[0] = make_float2(pt[q].x, pt[q].y);
+                to[1] = make_float2(pt[q].z, pt[q].w);
+            }
+        }
+    } else {
+        for (int e = tid; e < kKB * kKB; e += 256) {
+            const int r = e >> 6, c = e & 63;
+            sm.Dg[r][c] = ld_or_inf<kL2>(d, n, ld, K0 + r, K0 + c);
+            if (kind != 0) sm.T[r][c] = ld_or_inf<kL2>(d, n, ld, R0 + r, C0 + c);
+        }
     }
     __syncthreads();
     if (kind == 0 || !closed_diag) close_diag_blocked(sm.Dg);
@@ -265,15 +287,16 @@ __device__ __forceinline__ void fw_panel_tile(float* __restrict__ d, int n, int 
         }
 }
 
-// Update tile (ti, tj) of round kb, 128x128. 256 threads = 8 warps (4 x 2),
-// each warp 32 x 64, each thread 8 x 8 (rows/cols interleaved so the
-// shared-memory fragment loads are conflict-free 128-bit reads).
-template <bool kL2>
+// Update tile (ti, tj) of round kb, 128 x kCols. 256 threads = 8 warps (4 x 2),
+// each warp 32 x kCols / 2, each thread 8 x kCols / 16 (rows/cols interleaved so
+// the shared-memory fragment loads are conflict-free 128-bit reads).
+template <bool kL2, int kCols = kTile>
 __device__ __forceinline__ void fw_update_tile(float* __restrict__ d, int n, int ld, int kb, int ti, int tj,
                                                float2* __restrict__ As, float2* __restrict__ Bs) {
-    const int I0 = ti * kTile, J0 = tj * kTile, K0 = kb * kKB;
+    constexpr int kP = kCols / 32;  // column pairs a thread
+    const int I0 = ti * kTile, J0 = tj * kCols, K0 = kb * kKB;
     const int tid = threadIdx.x;
-    const bool full = (I0 + kTile <= n) && (J0 + kTile <= n) && (K0 + kKB <= n);
+    const bool full = (I0 + kTile <= n) && (J0 + kCols <= n) && (K0 + kKB <= n);
 
     // stage A = S[I0:I0+128, K0:K0+64] as k-pairs: As[kp][i] = {S[i][2kp], S[i][2kp+1]}
     {
@@ -296,12 +319,13 @@ __device__ __forceinline__ void fw_update_tile(float* __restrict__ d, int n, int
             As[(kp + 1) * (kTile + kApad) + i] = make_float2(v.z, v.w);
         }
     }
-    // stage B = S[K0:K0+64, J0:J0+128] as k-pairs: Bs[kp][j] = {S[2kp][j], S[2kp+1][j]}
+    // stage B = S[K0:K0+64, J0:J0+kCols] as k-pairs: Bs[kp][j] = {S[2kp][j], S[2kp+1][j]}
     {
-        const int j4 = tid & 31;
+        constexpr int kQ = kCols / 4;  // threads a row
+        const int j4 = tid % kQ;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int kp = (tid >> 5) + 8 * q;
+        for (int q = 0; q < 32 * kQ / 256; ++q) {
+            const int kp = tid / kQ + 256 / kQ * q;
             const int gk = K0 + 2 * kp, gj = J0 + 4 * j4;
             float4 r0, r1;
             if (full) {
@@ -313,7 +337,7 @@ __device__ __forceinline__ void fw_update_tile(float* __restrict__ d, int n, int
                 r1.x = ld_or_inf<kL2>(d, n, ld, gk + 1, gj); r1.y = ld_or_inf<kL2>(d, n, ld, gk + 1, gj + 1);
                 r1.z = ld_or_inf<kL2>(d, n, ld, gk + 1, gj + 2); r1.w = ld_or_inf<kL2>(d, n, ld, gk + 1, gj + 3);
             }
-            float4* dst = reinterpret_cast<float4*>(Bs + kp * kTile + 4 * j4);
+            float4* dst = reinterpret_cast<float4*>(Bs + kp * kCols + 4 * j4);
             dst[0] = make_float4(r0.x, r1.x, r0.y, r1.y);
             dst[1] = make_float4(r0.z, r1.z, r0.w, r1.w);
         }
@@ -322,16 +346,16 @@ __device__ __forceinline__ void fw_update_tile(float* __restrict__ d, int n, int
     const int warp = tid >> 5, lane = tid & 31;
     const int wy = warp >> 1, wx = warp & 1, ty = lane >> 3, tx = lane & 7;
     const int rbase = wy * 32 + ty * 2;  // rows rbase + 8q + {0,1}
-    const int cbase = wx * 64 + tx * 2;  // cols cbase + 16p + {0,1}
+    const int cbase = wx * (kCols / 2) + tx * 2;  // cols cbase + 16p + {0,1}
 
-    float acc[8][8];
+    float acc[8][2 * kP];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
             const int gi = I0 + rbase + 8 * q + s;
 #pragma unroll
-            for (int p = 0; p < 4; ++p) {
+            for (int p = 0; p < kP; ++p) {
                 const int gj = J0 + cbase + 16 * p;
                 float2 v;
                 if (full) {
@@ -349,14 +373,17 @@ __device__ __forceinline__ void fw_update_tile(float* __restrict__ d, int n, int
 
 #pragma unroll 1
     for (int kp = 0; kp < 32; ++kp) {
-        float2 a[8], b[8];
+        float2 a[8], b[2 * kP];
         const float4* ap = reinterpret_cast<const float4*>(As + kp * (kTile + kApad) + rbase);
-        const float4* bp = reinterpret_cast<const float4*>(Bs + kp * kTile + cbase);
+        const float4* bp = reinterpret_cast<const float4*>(Bs + kp * kCols + cbase);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const float4 va = ap[4 * q];   // rows rbase + 8q, +1
             a[2 * q] = make_float2(va.x, va.y);
             a[2 * q + 1] = make_float2(va.z, va.w);
+        }
+#pragma unroll
+        for (int q = 0; q < kP; ++q) {
             const float4 vb = bp[8 * q];   // cols cbase + 16q, +1
             b[2 * q] = make_float2(vb.x, vb.y);
             b[2 * q + 1] = make_float2(vb.z, vb.w);
@@ -364,7 +391,7 @@ __device__ __forceinline__ void fw_update_tile(float* __restrict__ d, int n, int
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
+            for (int c = 0; c < 2 * kP; ++c) {
                 const float2 s = __fadd2_rn(a[r], b[c]);
                 acc[r][c] = min3f(acc[r][c], s.x, s.y);
             }
@@ -379,7 +406,7 @@ __device__ __forceinline__ void fw_update_tile(float* __restrict__ d, int n, int
             const int gi = I0 + rbase + 8 * q + s;
             if (gi >= n || (gi >= K0 && gi < K0 + kKB)) continue;
 #pragma unroll
-            for (int p = 0; p < 4; ++p) {
+            for (int p = 0; p < kP; ++p) {
                 const int gj = J0 + cbase + 16 * p;
                 const bool okx = gj < n && !(gj >= K0 && gj < K0 + kKB);
                 const bool oky = gj + 1 < n && !(gj + 1 >= K0 && gj + 1 < K0 + kKB);
@@ -398,31 +425,39 @@ __device__ __forceinline__ void fw_update_tile(float* __restrict__ d, int n, int
 constexpr size_t kUpdateSmem = sizeof(float2) * 32 * (kTile + kApad) + sizeof(float2) * 32 * kTile;
 static_assert(sizeof(PanelSmem) <= kUpdateSmem, "panel tiles reuse the update stage");
 
-__global__ void __launch_bounds__(256) k_fw_panels(float* __restrict__ d, int n, int ld, int kb) {
+__global__ void __launch_bounds__(256) k_fw_panels(float* __restrict__ d, int n, int ld, int kb, int nt) {
     __shared__ PanelSmem sm;
-    fw_panel_tile<false>(d, n, ld, kb, blockIdx.x, sm);
+    fw_panel_tile<false>(d, n, ld, nt, kb, blockIdx.x, sm);
 }
 
+template <int kCols>
 __global__ void __launch_bounds__(256, 2) k_fw_update(float* __restrict__ d, int n, int ld, int kb) {
     extern __shared__ float4 fw_smem[];
     float2* As = reinterpret_cast<float2*>(fw_smem);
     float2* Bs = As + 32 * (kTile + kApad);
-    fw_update_tile<false>(d, n, ld, kb, blockIdx.y, blockIdx.x, As, Bs);
+    fw_update_tile<false, kCols>(d, n, ld, kb, blockIdx.y, blockIdx.x, As, Bs);
 }
 
-cudaError_t fw_solve(float* d, int n, int ld, cudaStream_t st) {
+cudaError_t fw_solve(float* d, int n, int ld, int padded, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    {
-        const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k_fw_update));
-        if (e != cudaSuccess) return e;
-    }
+    int sms = 0, dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = raise_smem_limit(reinterpret_cast<const void*>(k_fw_update<kTile>));
+    if (e == cudaSuccess) e = raise_smem_limit(reinterpret_cast<const void*>(k_fw_update<kTile / 2>));
+    if (e != cudaSuccess) return e;
     const int nt = (n + kKB - 1) / kKB;
     const int nu = (n + kTile - 1) / kTile;
+    // Tiles of 64 columns as long as each gets an SM of its own (n = 1021: 143
+    // against 233 us in 16 rounds, 64 tiles of 128 x 128 leave 88 SMs idle; n =
+    // 1300: 296 against 305, n = 2048: 844 against 747).
+    const bool narrow = nt * nu <= sms;
     for (int kb = 0; kb < nt; ++kb) {
-        k_fw_panels<<<2 * nt - 1, 256, 0, st>>>(d, n, ld, kb);
+        k_fw_panels<<<2 * nt - 1, 256, 0, st>>>(d, padded, ld, kb, nt);
         ++g_launch_counter;
         if (nt > 1) {
-            k_fw_update<<<dim3(nu, nu), 256, kUpdateSmem, st>>>(d, n, ld, kb);
+            if (narrow) k_fw_update<kTile / 2><<<dim3(nt, nu), 256, kUpdateSmem, st>>>(d, padded, ld, kb);
+            else k_fw_update<kTile><<<dim3(nu, nu), 256, kUpdateSmem, st>>>(d, padded, ld, kb);
             ++g_launch_counter;
         }
     }
@@ -567,7 +602,7 @@ __global__ void __launch_bounds__(256, 2) k_fw_persistent(float* __restrict__ ba
         if (s_abort) break;
         float* d = base + g.off;
         if (w.z == 0) {
-            fw_panel_tile<true>(d, g.n, g.ld, r, w.w, psm, /*closed_diag=*/true);
+            fw_panel_tile<true>(d, g.n, g.ld, nt, r, w.w, psm, /*closed_diag=*/true);
         } else {
             fw_update_tile<true>(d, g.n, g.ld, r, w.w / g.nu, w.w % g.nu, As, Bs);
         }

@@ -83,8 +83,9 @@ cudaError_t launch_paths(const float* pts, const GraphInfo* graphs, int n_graphs
 cudaError_t launch_edge_depths(const GraphInfo* graphs, int n_graphs, int max_edges, const int2* edges,
                                const int32_t* edge_cnt, const float* S, float* W, cudaStream_t st);
 
-// Floyd-Warshall on one matrix (general, any n, ld % 4 == 0).
-cudaError_t fw_solve(float* d, int n, int ld, cudaStream_t st);
+// Floyd-Warshall on one matrix (general, any n, ld % 4 == 0) of `padded` >= n
+// rows and columns, inf from n on: whole tiles take no bounds checks.
+cudaError_t fw_solve(float* d, int n, int ld, int padded, cudaStream_t st);
 
 // Path-solve schedules (lg_set_fw_schedule): 0 .. kFwSchedules - 1.
 constexpr int kFwSchedules = 6;
