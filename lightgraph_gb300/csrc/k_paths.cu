@@ -33,9 +33,9 @@
 // meet in the same banks 1.5 (K = 16) to ~2.6 times (K = 4), and by the barriers
 // of the passes where a graph is small; summing the lost fractions takes a
 // sixth of the time. Against the symmetric Floyd-Warshall with its fill and
-// mirror, edges and mirror included: 200 points 0.11 -> 0.055 ms, 1024 points
-// 0.41 -> 0.15 ms, 2500 points 1.00 -> 0.77 ms, 4096 points 2.72 -> 2.12 ms, 8
-// graphs of 4096 points 21.7 -> 11.6 ms, 24 of 2500 points 17.1 -> 10.7 ms.
+// mirror, preparation and mirror included: 200 points 0.055 against 0.11 ms, 1024
+// points 0.15 against 0.38 ms, 2500 points 0.77 against 0.95 ms, 4096 points 2.12
+// against 2.53 ms, 8 graphs of 4096 points 11.6 against 19.7 ms.
 #include <algorithm>
 
 #include "lg_kernels.h"

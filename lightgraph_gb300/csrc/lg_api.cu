@@ -963,14 +963,14 @@ bool Ctx::marched_as_set() const {
 // Floyd-Warshall solves the graphs where a schedule is pinned, a graph is too
 // large for shared memory or has too many edges, depths could be negative (only
 // a negative cutoff lets them through), a channel does not absorb, and in
-// batches that fill the GPU with it: it takes 0.4 us a point of the largest
-// graph or, if that is more, 1 ms for 2.4e10 (i, j, k); the solve from the edges
-// 1 ms for 1.1e7 (i, j), a little less for many graphs (16 of 500 points: 0.24
-// against 0.30 ms, 48 of 750: 1.34 against 1.53, 4 of 1500: 0.77 against 0.81,
-// but 2 of 2100: 1.00 against 0.87, 8 of 2500: 5.8 against 4.1); up to 2048
-// points a graph that is hardly ever less, and they are left to the autotuner.
+// batches that fill the GPU with it: it takes 0.38 us a point of the largest
+// graph or, if that is more, 1 ms for 2.6e10 (i, j, k); the solve from the edges
+// 1 ms for 1.2e7 (i, j) (16 of 500 points: 0.21 against 0.30 ms, 48 of 750: 1.09
+// against 1.53, 4 of 1500: 0.70 against 0.81, but 8 of 2500: 5.1 against 4.1, 8
+// of 4096: 19.5 against 11.6); up to 2048 points a graph that is hardly ever
+// less, and they are left to the autotuner.
 // Few and small ones leave both at their latency, which is shorter from the edges (8 of 200
-// points: 0.13 against 0.075 ms, 4 of 1000: 0.43 against 0.35).
+// points: 0.12 against 0.075 ms, 4 of 1000: 0.40 against 0.35).
 bool Ctx::path_unit(PathUnit& pu) const {
     if (fw_pinned >= 0 || settings.cutoff < 0.0 || max_n > kPathMaxPoints || max_connect > 16) return false;
     const bool few = n_graphs == 1 || (n_graphs <= 8 && n_points <= 4096);
@@ -981,7 +981,7 @@ bool Ctx::path_unit(PathUnit& pu) const {
             pairs += (double)g.n * g.n;
             triples += (double)g.ld * g.ld * g.ld;
         }
-        if (pairs / 1.1e7 >= std::max(4e-4 * max_n, triples / 2.4e10)) return false;
+        if (pairs / 1.2e7 >= std::max(3.8e-4 * max_n, triples / 2.6e10)) return false;
     }
     double a[3], lo = INFINITY, hi = 0.0;
     for (int c = 0; c < 3; ++c) {
