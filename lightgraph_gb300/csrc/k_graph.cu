@@ -76,13 +76,13 @@ __global__ void __launch_bounds__(256) k_candidates(const float* __restrict__ pt
 }
 
 // Whether a graph of n points whose candidate counts add up to sum is decided
-// by sweeps. Row by row the edges take ~0.21 us a point; sweeps take a chain
+// by sweeps. Row by row the edges take ~0.124 us a point; sweeps take a chain
 // of pairs that wait for one another, about as long as the neighbourhood of
 // twice the radius (8 partner counts), at ~0.7 us each, and ~20 us to start:
-// 4096 points with 22 partners 0.84 against 0.13 ms; 3531 points with 160
-// partners 0.72 against 1.3 ms.
+// 4096 points with 22 partners 0.51 against 0.13 ms; 3531 points with 160
+// partners 0.44 against 1.3 ms.
 __device__ __forceinline__ bool sweep_form(int n, int32_t sum) {
-    return sum < (1 << 20) && (int64_t)n * (n - 100) > 27 * 2 * (int64_t)sum;
+    return sum < (1 << 20) && (int64_t)n * (n - 160) > 45 * 2 * (int64_t)sum;
 }
 
 // One CTA per graph. Candidate rows are staged into shared memory in chunks
@@ -138,24 +138,49 @@ __global__ void __launch_bounds__(256) k_greedy(const float* __restrict__ pts,
                 greedy_stage(g, cand, cand_cnt, r1, min(kGreedyChunk, n - r1), cs2 + (buf ^ 1) * kGreedyChunk * kCandCap,
                              cc2 + (buf ^ 1) * kGreedyChunk, threadIdx.x - 32, blockDim.x - 32);
         } else {
+            // A row's candidates do not depend on the edge counts: its count and
+            // first 64 are loaded during the row before, and both batches are
+            // decided without a branch, so that the chain of a row is the loads
+            // of the counts, two ballots and the update (1024 points with 90
+            // partners: 213 -> 127 us; 32 graphs of 257 to 3805: 724 -> 436 us).
+            const unsigned below = (1u << lane) - 1u;
+            int next_total = cc[0], next_a = cs[lane], next_b = cs[32 + lane];
             for (int r = 0; r < rows; ++r) {
                 const int i = r0 + r;
-                // the row's candidate count and first 32 candidates do not
-                // depend on the edge counts: loaded beside cnt[i]
-                const int total = cc[r];
-                const int jfirst = cs[r * kCandCap + lane];
-                int need = max_connect - (int)cnt[i];
-                if (need <= 0) continue;
+                const int total = next_total, ja = next_a, jb = next_b;
+                const int rn = min(r + 1, rows - 1);
+                next_total = cc[rn];
+                next_a = cs[rn * kCandCap + lane];
+                next_b = cs[rn * kCandCap + 32 + lane];
                 const int stored = min(total, kCandCap);
-                for (int b = 0; b < stored && need > 0; b += 32) {
-                    const int c = b + lane;
-                    int j = -1;
-                    if (c < stored) j = b == 0 ? jfirst : cs[r * kCandCap + c];
-                    const bool elig = j >= 0 && (int)cnt[j] < max_connect;
-                    const unsigned m = __ballot_sync(0xffffffffu, elig);
-                    const int rank = __popc(m & ((1u << lane) - 1u));
-                    if (elig && rank < need) {
-                        cnt[j] = cnt[j] + 1;
+                const int ci = cnt[i];
+                const int ca = lane < stored ? (int)cnt[ja] : max_connect;
+                const int cb = 32 + lane < stored ? (int)cnt[jb] : max_connect;
+                int need = max(max_connect - ci, 0);
+                const unsigned ma = __ballot_sync(0xffffffffu, ca < max_connect);
+                const unsigned mb = __ballot_sync(0xffffffffu, cb < max_connect);
+                const int ra = __popc(ma & below), rb = __popc(ma) + __popc(mb & below);
+                if (ca < max_connect && ra < need) {
+                    cnt[ja] = (uint8_t)(ca + 1);
+                    E[ecount + ra] = make_int2(i, ja);
+                }
+                if (cb < max_connect && rb < need) {
+                    cnt[jb] = (uint8_t)(cb + 1);
+                    E[ecount + rb] = make_int2(i, jb);
+                }
+                const int got = min(__popc(ma) + __popc(mb), need);
+                need -= got;
+                ecount += got;
+                __syncwarp();
+                if (need == 0 || stored <= 64) continue;
+                static_assert(kCandCap == 96, "one more batch");
+                {
+                    const int j = 64 + lane < stored ? cs[r * kCandCap + 64 + lane] : 0;
+                    const int c = 64 + lane < stored ? (int)cnt[j] : max_connect;
+                    const unsigned m = __ballot_sync(0xffffffffu, c < max_connect);
+                    const int rank = __popc(m & below);
+                    if (c < max_connect && rank < need) {
+                        cnt[j] = (uint8_t)(c + 1);
                         E[ecount + rank] = make_int2(i, j);
                     }
                     const int acc = min(__popc(m), need);
@@ -167,22 +192,31 @@ __global__ void __launch_bounds__(256) k_greedy(const float* __restrict__ pts,
                     // more partners than stored: continue the scan past the last stored one
                     const int jstart = cs[r * kCandCap + kCandCap - 1] + 1;
                     const float pi[3] = {P[3 * i], P[3 * i + 1], P[3 * i + 2]};
-                    for (int j0 = jstart; j0 < n && need > 0; j0 += 32) {
-                        const int j = j0 + lane;
-                        bool elig = false;
-                        if (j < n) {
-                            const float pj[3] = {P[3 * j], P[3 * j + 1], P[3 * j + 2]};
-                            elig = pair_close(pi, pj, g.r2, lo, hi) && (int)cnt[j] < max_connect;
+                    for (int j0 = jstart; j0 < n && need > 0; j0 += 128) {
+                        // four batches: their loads and tests are independent
+                        bool elig[4];
+#pragma unroll
+                        for (int b = 0; b < 4; ++b) {
+                            const int j = j0 + 32 * b + lane;
+                            elig[b] = false;
+                            if (j < n) {
+                                const float pj[3] = {P[3 * j], P[3 * j + 1], P[3 * j + 2]};
+                                elig[b] = pair_close(pi, pj, g.r2, lo, hi) && (int)cnt[j] < max_connect;
+                            }
                         }
-                        const unsigned m = __ballot_sync(0xffffffffu, elig);
-                        const int rank = __popc(m & ((1u << lane) - 1u));
-                        if (elig && rank < need) {
-                            cnt[j] = cnt[j] + 1;
-                            E[ecount + rank] = make_int2(i, j);
+#pragma unroll
+                        for (int b = 0; b < 4; ++b) {
+                            const int j = j0 + 32 * b + lane;
+                            const unsigned m = __ballot_sync(0xffffffffu, elig[b]);
+                            const int rank = __popc(m & below);
+                            if (elig[b] && rank < need) {
+                                cnt[j] = cnt[j] + 1;
+                                E[ecount + rank] = make_int2(i, j);
+                            }
+                            const int acc = min(__popc(m), need);
+                            need -= acc;
+                            ecount += acc;
                         }
-                        const int acc = min(__popc(m), need);
-                        need -= acc;
-                        ecount += acc;
                         __syncwarp();
                     }
                 }
