@@ -498,7 +498,7 @@ __global__ void k_edge_depths(const GraphInfo* __restrict__ graphs, const int2* 
 
 int path_stride(int max_connect) { return std::max(2, (max_connect + 1) / 2 * 2); }
 
-cudaError_t launch_paths(const float* pts, const GraphInfo* graphs, int n_graphs, int max_n, int64_t n_points,
+cudaError_t launch_paths(const float* pts, const GraphInfo* graphs, int n_graphs, int min_n, int max_n, int64_t n_points,
                          int max_connect, const int2* edges, const int32_t* edge_cnt, const float* W, const PathUnit& pu,
                          const PathScratch& ps, float* S, int sms, cudaStream_t st) {
     if (n_graphs == 0 || max_n == 0) return cudaSuccess;
@@ -524,7 +524,7 @@ cudaError_t launch_paths(const float* pts, const GraphInfo* graphs, int n_graphs
     static_assert(path_smem(n_max4, 16) <= most && path_smem(n_max2, 8) <= most && path_smem(kPathMaxPoints, 4) <= most);
     auto run = [&](auto pairs6, auto pairs, int K, int n_min, int n_max) {
         n_max = std::min(n_max, max_n);
-        if (e != cudaSuccess || n_max <= n_min) return;
+        if (e != cudaSuccess || n_max <= n_min || n_max < min_n) return;
         auto kernel = half == 6 ? pairs6 : pairs;
         if ((e = raise_smem_limit(reinterpret_cast<const void*>(kernel))) != cudaSuccess) return;
         kernel<<<dim3((n_max + K - 1) / K, n_graphs), n_max > kSmall ? 512 : 256, path_smem(n_max, K), st>>>(

@@ -1024,7 +1024,9 @@ lg_status Ctx::solve_from_edges(const PathUnit& pu) {
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "device query");
     const PathScratch ps = {d_path_order.as<uint16_t>(), d_path_order.as<uint16_t>() + P, d_path_ell.as<int4>(),
                             reinterpret_cast<uint32_t*>(d_path_ell.as<int2>() + places), d_path_step.as<uint32_t>()};
-    CK(launch_paths(d_pts.as<float>(), d_graphs.as<GraphInfo>(), n_graphs, max_n, n_points, max_connect,
+    int min_n = max_n;
+    for (const GraphInfo& g : h_graphs) min_n = std::min(min_n, g.n);
+    CK(launch_paths(d_pts.as<float>(), d_graphs.as<GraphInfo>(), n_graphs, min_n, max_n, n_points, max_connect,
                     d_edges.as<int2>(), d_edge_cnt.as<int32_t>(), d_edge_depth.as<float>(), pu, ps, d_S.as<float>(),
                     sms, st), "paths from the edges");
     return LG_OK;

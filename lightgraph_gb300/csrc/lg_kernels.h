@@ -75,7 +75,7 @@ struct PathScratch {
 };
 constexpr int kPathMaxPoints = 9200;  // K = 4 distances of a graph in shared memory
 int path_stride(int max_connect);
-cudaError_t launch_paths(const float* pts, const GraphInfo* graphs, int n_graphs, int max_n, int64_t n_points,
+cudaError_t launch_paths(const float* pts, const GraphInfo* graphs, int n_graphs, int min_n, int max_n, int64_t n_points,
                          int max_connect, const int2* edges, const int32_t* edge_cnt, const float* W, const PathUnit& pu,
                          const PathScratch& ps, float* S, int sms, cudaStream_t st);
 
