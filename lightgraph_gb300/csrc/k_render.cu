@@ -19,8 +19,12 @@
 //                      counting sort's scatter), so the rays in flight are
 //                      neighbouring, parallel rays;
 //   k_shadow         : one thread per (light, ordered pair of tasks) marches
-//                      that light's shadow rays (all its samples) and writes
-//                      the light's contribution to the task's slot;
+//                      that light's shadow rays and writes its contribution
+//                      to the task's slot;
+//   k_shadow_env     : the same for environment lights, whose rays go in
+//                      sampled directions; where there are many and the records
+//                      exceed L2, a light sample at a time, ordered by direction
+//                      and start cell (k_env_keys, a scan, k_env_scatter);
 //   k_resolve        : per pixel, sums the tasks and lights in order and
 //                      writes the films.
 // Shadow rays accumulate a scalar optical depth (every channel of the
