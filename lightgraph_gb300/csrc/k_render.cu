@@ -311,7 +311,7 @@ struct PixelSample {
 // which samples shade (positions, transmittance, termination, step jitter)
 // is spelled out rounding by rounding (no contraction left to the compiler).
 // Returns the primary samples taken.
-template <bool kWrite, int DT>
+template <bool kWrite, int DT, bool kAhead>
 __device__ __forceinline__ uint32_t primary_sample(const DevScene& sc, const DevCamera& cam, const DevScatterGrid& sg,
                                                    int64_t ps, int32_t* __restrict__ counts,
                                                    const int32_t* __restrict__ offsets, ShadowTask* __restrict__ tasks,
@@ -339,18 +339,43 @@ __device__ __forceinline__ uint32_t primary_sample(const DevScene& sc, const Dev
             float pStep = jitter_step(step0, draw(stream, kTagPrimarySpan | span_ord));
             ++span_ord;
             // (pT + pStep > pT stops a march whose step underflows against pT)
-            for (float pT = step0 * ceilf(ta / step0); pT <= tb && pT + pStep > pT;) {
+            RawCell<DT> cell;  // kAhead: the record under pT
+            float wx, wy, wz;
+            float pT = step0 * ceilf(ta / step0);
+            auto load = [&] {
+                cell = ld_raw<DT>(G.data, span_cell(G, __fmaf_rn(pT, pr.d[0], pr.e[0]), __fmaf_rn(pT, pr.d[1], pr.e[1]),
+                                                    __fmaf_rn(pT, pr.d[2], pr.e[2]), wx, wy, wz));
+            };
+            if (kAhead && pT <= tb) load();
+            while (pT <= tb && pT + pStep > pT) {
                 const uint32_t n = n_iter++;
                 jit = step_next(jit);
                 ++n_primary;
                 const float p[3] = {__fmaf_rn(pT, pr.d[0], pr.e[0]), __fmaf_rn(pT, pr.d[1], pr.e[1]),
                                     __fmaf_rn(pT, pr.d[2], pr.e[2])};
-                const float rho = fminf(sample_span_t<DT>(G, p[0], p[1], p[2]) * sh.dS, sh.dMax);
-                if (rho < cutoff) { pT += pStep; continue; }
+                float raw;
+                if (kAhead) {
+                    float v[8];
+                    decode_cell<DT>(cell, v);
+                    raw = record_sample<DT>(v, wx, wy, wz);
+                } else {
+                    raw = sample_span_t<DT>(G, p[0], p[1], p[2]);
+                }
+                const float rho = fminf(raw * sh.dS, sh.dMax);
+                const float taken = pStep;
+                if (kAhead) {  // the next sample's place is settled: its record comes in beside this one's shading
+                    if (!(rho < cutoff)) pStep = jitter_step_bits(step0, jit);
+                    pT += pStep;
+                    if (pT <= tb) load();
+                    if (rho < cutoff) continue;
+                } else if (rho < cutoff) {
+                    pT += pStep;
+                    continue;
+                }
                 float omdT[3], dT[3];
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
-                    const float e1 = expm1_approx(-sh.a[c] * rho * pStep);
+                    const float e1 = expm1_approx(-sh.a[c] * rho * taken);
                     dT[c] = 1.f + e1;
                     omdT[c] = -e1;
                 }
@@ -385,6 +410,10 @@ __device__ __forceinline__ uint32_t primary_sample(const DevScene& sc, const Dev
                                 if (k >= ko.rb.n) break;
                                 const uint32_t key = ray_key(ko.rb.b[k], p);
                                 ko.keys[k * ko.unit_cap + u] = key;
+                                if (kAhead) {
+                                    atomicAdd(ko.key_counts + key, 1);
+                                    continue;
+                                }
                                 // lanes filing under the same key share one atomic
                                 const cg::coalesced_group grp = cg::labeled_partition(cg::coalesced_threads(), key);
                                 if (grp.thread_rank() == 0) atomicAdd(ko.key_counts + key, (int)grp.size());
@@ -404,8 +433,10 @@ __device__ __forceinline__ uint32_t primary_sample(const DevScene& sc, const Dev
                     pdrop = true;
                     break;
                 }
-                pStep = jitter_step_bits(step0, jit);
-                pT += pStep;
+                if (!kAhead) {
+                    pStep = jitter_step_bits(step0, jit);
+                    pT += pStep;
+                }
             }
         }
     }
@@ -419,12 +450,18 @@ __device__ __forceinline__ uint32_t primary_sample(const DevScene& sc, const Dev
     return n_primary;
 }
 
+// kAhead, for images of so few rays that the chain of each is what takes the
+// time: the next sample's record is on its way while this one is shaded, and
+// lanes count their order keys one by one (seldom are two alike); the registers
+// that takes leave room for 4 CTAs.
+constexpr int kAheadCtas = 4;
+
 // Warps claim 32 consecutive pixel samples at a time from *claim (zero at
 // launch) until none are left: a persistent grid in which no warp slot waits
 // on another warp's long ray. The shading pass runs 5 CTAs per SM so that
 // its registers do not spill; the count pass, lighter, runs 6.
-template <bool kWrite, int DT>
-__global__ void __launch_bounds__(128, kWrite ? 5 : 6) k_primary(DevScene sc, DevCamera cam, DevScatterGrid sg,
+template <bool kWrite, int DT, bool kAhead = false>
+__global__ void __launch_bounds__(128, kAhead ? kAheadCtas : kWrite ? 5 : 6) k_primary(DevScene sc, DevCamera cam, DevScatterGrid sg,
                                                  int32_t* __restrict__ counts, const int32_t* __restrict__ offsets,
                                                  ShadowTask* __restrict__ tasks, int64_t task_cap,
                                                  PixelSample* __restrict__ out, unsigned long long* __restrict__ ctr,
@@ -442,7 +479,7 @@ __global__ void __launch_bounds__(128, kWrite ? 5 : 6) k_primary(DevScene sc, De
         if ((int64_t)claimed >= n_ps) break;
         const int64_t ps = (int64_t)claimed + lane;
         if (ps < n_ps)
-            n_primary += primary_sample<kWrite, DT>(sc, cam, sg, ps, counts, offsets, tasks, task_cap, out, ko);
+            n_primary += primary_sample<kWrite, DT, kAhead>(sc, cam, sg, ps, counts, offsets, tasks, task_cap, out, ko);
     }
     if (kWrite && ctr) {
         unsigned long long q = n_primary;
@@ -1094,8 +1131,12 @@ cudaError_t launch_render_shade(const DevScene& sc, const DevCamera& cam, const 
     const int64_t n_pix = (int64_t)cam.width * cam.height;
     if (n_ps == 0) return cudaSuccess;
     PixelSample* pss = reinterpret_cast<PixelSample*>(pixel_samples);
-    const unsigned blocks = (unsigned)std::min<int64_t>((n_ps + 127) / 128,
-                                                        (int64_t)sms * primary_ctas_per_sm(true, sc.dens.dtype));
+    // Up to two waves of the form that fetches a record ahead: 121 x 89 pixel
+    // samples 80 -> 67 us, 256^2 114 -> 103 us, 480 x 270 293 -> 258 us; 411 x 307
+    // at 2 spp either way, 1024^2 at 4 spp 4.17 against 4.28 ms.
+    const bool ahead = (n_ps + 127) / 128 <= 2ll * kAheadCtas * sms;
+    const unsigned blocks = (unsigned)std::min<int64_t>(
+        (n_ps + 127) / 128, (int64_t)sms * (ahead ? kAheadCtas : primary_ctas_per_sm(true, sc.dens.dtype)));
     auto mark = [&](int k) {
         if (marks && marks[k]) cudaEventRecord(marks[k], st);
     };
@@ -1104,15 +1145,12 @@ cudaError_t launch_render_shade(const DevScene& sc, const DevCamera& cam, const 
     // keys and counts them (the counts zeroed first)
     if (ro.rb.n > 0 && (e = cudaMemsetAsync(ro.key_counts, 0, sizeof(int32_t) * ro.n_keys, st)) != cudaSuccess)
         return e;
-    if (sc.dens.dtype == 1)
-        k_primary<true, 1><<<blocks, 128, 0, st>>>(sc, cam, sg, nullptr, offsets, tasks, task_cap, pss, counters,
-                                                   counters + 4, ro, 0);
-    else if (sc.dens.dtype == 2)
-        k_primary<true, 2><<<blocks, 128, 0, st>>>(sc, cam, sg, nullptr, offsets, tasks, task_cap, pss, counters,
-                                                   counters + 4, ro, 0);
-    else
-        k_primary<true, 0><<<blocks, 128, 0, st>>>(sc, cam, sg, nullptr, offsets, tasks, task_cap, pss, counters,
-                                                   counters + 4, ro, 0);
+    auto shade = [&](auto kernel) {
+        kernel<<<blocks, 128, 0, st>>>(sc, cam, sg, nullptr, offsets, tasks, task_cap, pss, counters, counters + 4, ro, 0);
+    };
+    if (sc.dens.dtype == 1) shade(ahead ? k_primary<true, 1, true> : k_primary<true, 1, false>);
+    else if (sc.dens.dtype == 2) shade(ahead ? k_primary<true, 2, true> : k_primary<true, 2, false>);
+    else shade(ahead ? k_primary<true, 0, true> : k_primary<true, 0, false>);
     ++g_launch_counter;
     mark(0);
     // order the shadow rays: scan the key counts, scatter the units

@@ -90,27 +90,49 @@ __host__ __device__ inline void cell_coefs(const float v[8], float c[8]) {
     c[7] = (dxyz - dxz) - (dyz - dz);
 }
 
-// The raw eight values of record rec, decoded to FP32 (FP16/BF16: voxel
-// values in a + 2b + 4c order; FP32: cell_coefs).
+// A record as it is stored.
 template <int DT>
-__device__ __forceinline__ void ld_cell(const void* data, uint32_t rec, float v[8]) {
-    if (DT == 0) {
-        const float* p = reinterpret_cast<const float*>(data) + (size_t)rec * 8;
-        asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-            : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+struct RawCell {
+    uint32_t w[DT == 0 ? 8 : 4];
+};
+template <int DT>
+__device__ __forceinline__ RawCell<DT> ld_raw(const void* data, uint32_t rec) {
+    RawCell<DT> c;
+    if constexpr (DT == 0) {
+        const uint32_t* p = reinterpret_cast<const uint32_t*>(data) + (size_t)rec * 8;
+        asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=r"(c.w[0]), "=r"(c.w[1]), "=r"(c.w[2]), "=r"(c.w[3]), "=r"(c.w[4]), "=r"(c.w[5]), "=r"(c.w[6]), "=r"(c.w[7])
             : "l"(p));
     } else {
         const uint4 q = __ldg(reinterpret_cast<const uint4*>(data) + rec);
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+        c.w[0] = q.x;
+        c.w[1] = q.y;
+        c.w[2] = q.z;
+        c.w[3] = q.w;
+    }
+    return c;
+}
+// Its eight values in FP32 (FP16/BF16: voxel values in a + 2b + 4c order; FP32:
+// cell_coefs).
+template <int DT>
+__device__ __forceinline__ void decode_cell(const RawCell<DT>& c, float v[8]) {
+    if constexpr (DT == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(c.w[i]);
+    } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             float2 f;
-            if (DT == 1) f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-            else f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+            if (DT == 1) f = __half22float2(*reinterpret_cast<const __half2*>(&c.w[i]));
+            else f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&c.w[i]));
             v[2 * i] = f.x;
             v[2 * i + 1] = f.y;
         }
     }
+}
+template <int DT>
+__device__ __forceinline__ void ld_cell(const void* data, uint32_t rec, float v[8]) {
+    decode_cell<DT>(ld_raw<DT>(data, rec), v);
 }
 
 // Record index of cell (ix, iy, iz), or 0 (the all-zero padding cell) when
