@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(128) k_edge_march(DevScene sc, const float* __
         float tau;
         bool dropped;
         uint32_t ns = 0;
-        if (march_fixed<DT>(G, r, sc.step1, scale, sh.dMax, sh.tau_drop, contrib, tau, dropped, ns)) {
+        if (march_fixed<DT, 1>(G, r, sc.step1, scale, sh.dMax, sh.tau_drop, contrib, tau, dropped, ns)) {
             value = dropped ? kInf : tau;
         }
     }
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(128) k_vertex_light(DevScene sc, const float* 
             bool dropped;
             uint32_t nsmp = 0;
             // a ray that misses the grid bbox or drops out adds nothing
-            if (march_fixed<DT>(G0, ray, sc.step1, scale, sh.dMax, sh.tau_drop, contrib, tau, dropped, nsmp) &&
+            if (march_fixed<DT, 4>(G0, ray, sc.step1, scale, sh.dMax, sh.tau_drop, contrib, tau, dropped, nsmp) &&
                 !dropped) {
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {

@@ -613,9 +613,13 @@ __device__ __forceinline__ void illuminate(const DevLight& L, const float p[3], 
 //   tau = sum over samples of contrib(rho) * step,
 // where rho = min(sample * scale, densityMax) and contrib() is given by the
 // caller. Returns false if the ray misses the leaf bbox. Sets dropped when
-// tau crosses sh.tau_drop (the reference's |T|^2 < cutoff test).
+// tau crosses sh.tau_drop (the reference's |T|^2 < cutoff test). The places of the
+// samples do not depend on what they read: kMarchAhead records are fetched at
+// once. Vertex light takes 4 (4096 points, two lights: 75 -> 44 us; 48 clouds of
+// 750: 77 -> 53 us); for the edges, of which there are more and which are short,
+// it does not pay (48 clouds: 27 us with 1, 29 with 2 or 4).
 // ---------------------------------------------------------------------------
-template <int DT, class Contrib>
+template <int DT, int kMarchAhead, class Contrib>
 __device__ __forceinline__ bool march_fixed(const DevGrid& g, IRay r, float step, float scale,
                                             float dmax, float tau_drop, Contrib contrib,
                                             float& tau, bool& dropped, uint32_t& nsamples) {
@@ -626,15 +630,32 @@ __device__ __forceinline__ bool march_fixed(const DevGrid& g, IRay r, float step
     dda_init(s, r, g);
     float ta, tb;
     while (next_span_flat(g, s, ta, tb)) {
-        for (float t = step * ceilf(ta / step); t <= tb && t + step > t; t += step) {
-            const float rho = fminf(
-                sample_index_t<DT>(g, r.e[0] + t * r.d[0], r.e[1] + t * r.d[1], r.e[2] + t * r.d[2]) * scale,
-                dmax);
-            ++nsamples;
-            float c;
-            if (!contrib(rho, c)) continue;
-            tau += c * step;
-            if (tau > tau_drop) { dropped = true; return true; }
+        for (float t = step * ceilf(ta / step); t <= tb && t + step > t;) {
+            // kMarchAhead records at once (past the span's end the padding record)
+            RawCell<DT> cell[kMarchAhead];
+            float w[kMarchAhead][3], tk = t;
+#pragma unroll
+            for (int k = 0; k < kMarchAhead; ++k, tk += step) {
+                const float p[3] = {r.e[0] + tk * r.d[0], r.e[1] + tk * r.d[1], r.e[2] + tk * r.d[2]};
+                const float f[3] = {floorf(p[0]), floorf(p[1]), floorf(p[2])};
+                const uint32_t rec = cell_record(g, (int)f[0], (int)f[1], (int)f[2]);
+                cell[k] = ld_raw<DT>(g.data, tk <= tb ? rec : 0u);
+#pragma unroll
+                for (int a = 0; a < 3; ++a) w[k][a] = p[a] - f[a];
+            }
+#pragma unroll
+            for (int k = 0; k < kMarchAhead; ++k) {
+                if (!(t <= tb && t + step > t)) break;
+                float v[8];
+                decode_cell<DT>(cell[k], v);
+                const float rho = fminf(record_sample<DT>(v, w[k][0], w[k][1], w[k][2]) * scale, dmax);
+                t += step;
+                ++nsamples;
+                float c;
+                if (!contrib(rho, c)) continue;
+                tau += c * step;
+                if (tau > tau_drop) { dropped = true; return true; }
+            }
         }
     }
     return true;
