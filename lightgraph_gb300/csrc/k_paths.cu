@@ -33,9 +33,9 @@
 // meet in the same banks 1.5 (K = 16) to ~2.6 times (K = 4), and by the barriers
 // of the passes where a graph is small; summing the lost fractions takes a
 // sixth of the time. Against the symmetric Floyd-Warshall with its fill and
-// mirror, preparation and mirror included: 200 points 0.055 against 0.11 ms, 1024
-// points 0.15 against 0.38 ms, 2500 points 0.77 against 0.95 ms, 4096 points 2.12
-// against 2.53 ms, 8 graphs of 4096 points 11.6 against 19.7 ms.
+// mirror, preparation and mirror included: 200 points 0.051 against 0.10 ms, 1024
+// points 0.15 against 0.37 ms, 2500 points 0.74 against 0.93 ms, 4096 points 2.04
+// against 2.53 ms, 8 graphs of 4096 points 11.0 against 19.7 ms.
 #include <algorithm>
 
 #include "lg_kernels.h"
@@ -65,7 +65,19 @@ __device__ __forceinline__ uint32_t spread_bits4(uint32_t v) {
 // and what the units from there are off by, in fractions that (n - 1) edges
 // each off by a whole unit cannot overflow.
 __device__ __forceinline__ uint32_t path_word(int place, int rest) { return ((uint32_t)place << 18) | ((uint32_t)rest & 0x3FFFFu); }
-__device__ __forceinline__ int path_fraction(int n) { return 1 << min(10, 17 - (32 - __clz(n - 1))); }
+__device__ __forceinline__ int path_fraction_bits(int n) { return min(10, 17 - (32 - __clz(n - 1))); }
+
+// Depth w in 2^-bits units, to the nearest: w's 24 bits times the 64 of pu.per.
+// Integers, since FP64 runs at 1/64 of their rate (with it here and where the
+// distances are handed out, 32 graphs of 257 to 3805 points took 8.00 ms, not 7.76).
+__device__ __forceinline__ uint64_t path_units(const PathUnit& pu, float w, int bits) {
+    const uint32_t b = __float_as_uint(w) & 0x7FFFFFFFu;
+    const int e = max((int)(b >> 23), 1);
+    const uint64_t m = (b & 0x7FFFFFu) | (b >> 23 ? 0x800000u : 0u);
+    const uint64_t v = m * (uint32_t)(pu.per >> 32) + ((m * (uint32_t)pu.per) >> 32);
+    const int s = 182 - e - pu.exponent - bits;  // at least 12: the result stays below 2^43
+    return s > 63 ? 0 : (v + (1ull << (s - 1))) >> s;
+}
 
 __global__ void __launch_bounds__(kPrepThreads) k_path_prep(const float* __restrict__ pts,
                                                             const GraphInfo* __restrict__ graphs,
@@ -163,25 +175,34 @@ __global__ void __launch_bounds__(kPrepThreads) k_path_prep(const float* __restr
     int2* row = reinterpret_cast<int2*>(ell) + g.pt_off * stride;
     uint32_t* off = rest + g.pt_off * stride;
     const int ne = edge_cnt[blockIdx.x];
-    const double fraction = path_fraction(n);
+    const int bits = path_fraction_bits(n);
     unsigned long long sum = 0;
     int cnt = 0;
-    for (int e = tid; e < ne; e += kPrepThreads) {
-        const float w = W[g.e_off + e];
-        if (!(w <= pu.longest)) continue;  // dropped, or past the last depth that matters
-        const double units = (double)w * pu.per_unit;
-        const int d = (int)max(1u, __double2uint_rn(units));
-        const int lost = __double2int_rn((units - (double)(unsigned)d) * fraction);
-        const int2 ij = edges[g.e_off + e];
-        const int a = place[ij.x], b = place[ij.y];
-        const int ka = atomicAdd(deg + a, 1), kb = atomicAdd(deg + b, 1);
-        const int64_t ia = ((int64_t)(ka >> 1) * n + a) * 2 + (ka & 1), ib = ((int64_t)(kb >> 1) * n + b) * 2 + (kb & 1);
-        row[ia] = make_int2(b, d);
-        row[ib] = make_int2(a, d);
-        off[ia] = path_word(b, lost);
-        off[ib] = path_word(a, lost);
-        sum += (unsigned)d;
-        ++cnt;
+    for (int e0 = tid; e0 < ne; e0 += 4 * kPrepThreads) {
+        float ws[4];
+        int2 es[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {  // loads of four edges in flight
+            const int e = e0 + k * kPrepThreads;
+            ws[k] = e < ne ? W[g.e_off + e] : kInf;
+            es[k] = e < ne ? edges[g.e_off + e] : make_int2(0, 0);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (!(ws[k] <= pu.longest)) continue;  // dropped, or past the last depth that matters
+            const uint64_t units = path_units(pu, ws[k], bits);
+            const int d = (int)max(1u, (uint32_t)((units + ((1ull << bits) >> 1)) >> bits));
+            const int lost = (int)((int64_t)units - ((int64_t)(uint32_t)d << bits));
+            const int a = place[es[k].x], b = place[es[k].y];
+            const int ka = atomicAdd(deg + a, 1), kb = atomicAdd(deg + b, 1);
+            const int64_t ia = ((int64_t)(ka >> 1) * n + a) * 2 + (ka & 1), ib = ((int64_t)(kb >> 1) * n + b) * 2 + (kb & 1);
+            row[ia] = make_int2(b, d);
+            row[ib] = make_int2(a, d);
+            off[ia] = path_word(b, lost);
+            off[ib] = path_word(a, lost);
+            sum += (unsigned)d;
+            ++cnt;
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -410,8 +431,12 @@ __global__ void __launch_bounds__(1024) k_paths(const GraphInfo* __restrict__ gr
     const uint16_t* rk = rank + g.pt_off;
     const uint32_t* off = rest + g.pt_off * 2 * half;
     const uint32_t* dist = reinterpret_cast<const uint32_t*>(d);
-    const long long fraction = path_fraction(n);
-    const double scale = 1.0 / ((double)fraction * pu.per_unit);
+    // a distance of x = a 2^20 + b fractions in FP32, as c1 a + c0 b with the
+    // factors' second halves: off by little more than the one rounding
+    const int bits = path_fraction_bits(n);
+    const double scale = 1.0 / ((double)(1 << bits) * pu.per_unit);
+    const float c0 = (float)scale, c0_lo = (float)(scale - (double)c0);
+    const float c1 = (float)(scale * 1048576.0), c1_lo = (float)(scale * 1048576.0 - (double)c1);
     float* M = S + g.s_off;
     for (int k = 0; k < ns; ++k) {
         const int root = s0 + k;
@@ -453,7 +478,11 @@ __global__ void __launch_bounds__(1024) k_paths(const GraphInfo* __restrict__ gr
             if (j < n) {
                 const int v = rk[j];
                 const uint32_t m = dist[v * K + k], w = word[v];
-                if (m < far) out = (float)((double)(fraction * m + ((int)(w << 14) >> 14)) * scale);
+                if (m < far) {
+                    const int64_t x = ((int64_t)m << bits) + ((int)(w << 14) >> 14);
+                    const float a = (float)(uint32_t)(x >> 20), b = (float)(uint32_t)(x & 0xFFFFF);
+                    out = __fmaf_rn(a, c1, __fmaf_rn(b, c0, __fmaf_rn(a, c1_lo, __fmul_rn(b, c0_lo))));
+                }
             }
             row[j] = out;
         }

@@ -966,8 +966,8 @@ bool Ctx::marched_as_set() const {
 // batches that fill the GPU with it: it takes 0.38 us a point of the largest
 // graph or, if that is more, 1 ms for 2.6e10 (i, j, k); the solve from the edges
 // 1 ms for 1.2e7 (i, j) (16 of 500 points: 0.21 against 0.30 ms, 48 of 750: 1.09
-// against 1.53, 4 of 1500: 0.70 against 0.81, but 8 of 2500: 5.1 against 4.1, 8
-// of 4096: 19.5 against 11.6); up to 2048 points a graph that is hardly ever
+// against 1.53, 4 of 1500: 0.70 against 0.81, but 8 of 2500: 5.2 against 3.8, 8
+// of 4096: 19.7 against 11.0); up to 2048 points a graph that is hardly ever
 // less, and they are left to the autotuner.
 // Few and small ones leave both at their latency, which is shorter from the edges (8 of 200
 // points: 0.12 against 0.075 ms, 4 of 1000: 0.40 against 0.35).
@@ -995,6 +995,7 @@ bool Ctx::path_unit(PathUnit& pu) const {
     const double edge = std::min(R, 1.0001 * (double)std::max(dropout_depth(a, settings.cutoff), 0.f));
     if (!(edge > 0.0)) return false;  // every edge drops out
     pu.per_unit = 4294960000.0 / (R + edge);
+    pu.per = (uint64_t)std::ldexp(std::frexp(pu.per_unit, &pu.exponent), 64);
     pu.longest = (float)edge;
     pu.far = (uint32_t)(R * pu.per_unit);
     return true;

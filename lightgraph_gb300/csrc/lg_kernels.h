@@ -63,7 +63,9 @@ cudaError_t launch_vertex_light(const DevScene& sc, const float* pts, const Grap
 // Distances are counted in units: `far` of them and more are no path, and an
 // edge no longer than `longest` added to far still fits 32 bits.
 struct PathUnit {
-    double per_unit;
+    double per_unit;  // units in a depth of 1: per / 2^64 * 2^exponent
+    uint64_t per;
+    int exponent;
     float longest;
     uint32_t far;
 };
