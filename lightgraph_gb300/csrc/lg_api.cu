@@ -1937,6 +1937,7 @@ extern "C" lg_status lg_frame_device(lg_ctx* handle, int max_connect, double poi
     if (ctx->graph_valid && ctx->graph_epoch == g_alloc_epoch && ctx->graph_pvs == point_voxel_size &&
         std::memcmp(&ctx->graph_cam, camera, sizeof(lg_camera)) == 0) {
         CK(cudaGraphLaunch(ctx->graph_exec, ctx->st), "frame graph launch");
+        ctx->marched.valid = false;  // the replayed frame solves in the matrices
         ++g_launch_counter;
         ctx->ev_recorded = ctx->profiling;
         ctx->waves_recorded = ctx->profiling;

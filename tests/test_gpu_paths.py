@@ -71,3 +71,25 @@ def test_group_sizes(gpu_ctx, scene, sizes):
 @pytest.mark.parametrize("n", [5640, 5641, 9200, 9201])
 def test_largest_graphs(gpu_ctx, scene, n):
     solve(gpu_ctx, scene, [cloud(scene, n, 9)], [float(1.1 * n ** (-1.0 / 3.0))], 12, oracle=False)
+
+
+def test_matrix_of_other_settings(gpu_ctx, scene):
+    """Matrices marched under another cutoff or already solved keep to
+    Floyd-Warshall: the same bits as with a schedule pinned."""
+    import copy
+    other = copy.deepcopy(scene.opts)
+    other.cutoff = 0.02
+    out = {}
+    for schedule in (-1, 4):
+        scenes.load_into(gpu_ctx, scene)
+        gpu_ctx.set_fw_schedule(schedule)
+        gpu_ctx.build_graphs([cloud(scene, 300, 5)], [np.float32(0.2) ** 2], 12)
+        gpu_ctx.march_edges()
+        gpu_ctx.set_settings(other)
+        first = gpu_ctx.solve_paths(want=True)[0]
+        used, _ = gpu_ctx.fw_schedule()
+        out[schedule] = first, gpu_ctx.solve_paths(want=True)[0]
+        assert used >= 0
+    gpu_ctx.set_fw_schedule(-1)
+    for a, b in zip(out[-1], out[4]):
+        assert np.array_equal(a, b)
