@@ -623,14 +623,14 @@ struct DartFirst : DartTables<kDartChunk> {
     float x[kDartSlots][3][kDartChunk];
     uint32_t bits[kDartSlots][kDartChunk / 32];
     uint32_t ready[kDartSlots];
-    int queued[2], failed;  // failed: a helper did not answer
+    int queued[2];
     uint16_t queue[2][kDartChunk];
 };
 // Helpers. used: chunks that the first CTA is done with.
 struct DartHelper {
     uint32_t words[3][16 * kMtN];
     uint32_t used, stop;
-    int claim[2], quit;
+    int claim[2];
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -690,7 +690,6 @@ __device__ __forceinline__ void dart_helper(const DevGrid& g, const DartParams& 
         sh.used = 0;
         sh.stop = 0;
         sh.claim[0] = sh.claim[1] = 0;
-        sh.quit = 0;
     }
     cluster_sync();
     int buf = 2;
@@ -707,7 +706,6 @@ __device__ __forceinline__ void dart_helper(const DevGrid& g, const DartParams& 
             for (int k = 0; k < n; ++k) mt_next_chunk<16>(sh.words[(buf + k) % 3], sh.words[(buf + k + 1) % 3], twister);
         const int slot = c % kDartSlots;
         const bool free = c < kDartSlots || wait_for(&sh.used, c + 1 - kDartSlots, &sh.stop);
-        if (!free) sh.quit = 1;
         while (free) {
             int j = 0;
             if (lane == 0) j = atomicAdd(&sh.claim[par], 64);
@@ -726,8 +724,9 @@ __device__ __forceinline__ void dart_helper(const DevGrid& g, const DartParams& 
             }
         }
         asm volatile("fence.acq_rel.cluster;" ::: "memory");
-        __syncthreads();
-        if (sh.quit) break;
+        // all warps leave in the same round: the barrier itself carries the word,
+        // since a flag could be set for the next round while some still read it
+        if (__syncthreads_or(!free)) break;
         if (tid == 0) {
             sh.claim[par] = 0;  // used again in the chunk after next
             remote_release(remote(&first.ready[slot], 0), c + 1);
@@ -757,19 +756,16 @@ __global__ void __launch_bounds__(1024, 1) k_dart_cluster(DevGrid g, DartParams 
     clear_tables(sh, prm, tid, 1024);
     if (tid < kDartSlots) sh.ready[tid] = 0;
     if (tid < 2) sh.queued[tid] = 0;
-    if (tid == 0) sh.failed = 0;
+    bool failed = false;  // a helper did not answer; the same in every thread
     uint64_t boundary = prm.batch - 1u;
     uint32_t update = 0;
     if (tid == 0 && boundary == 0u) radius_update(sh.m2, 0, expected[0]);
     cluster_sync();
     // the hint tests of candidates [j0, j1) of the slot with chunk c, by the
-    // warps w of nw: those left go to the queue
+    // warps w of nw: those left go to the queue; false if the chunk did not come
     auto hint_tests = [&](uint32_t c, int j0, int j1, float hint_m2, int queue, int w, int nw) {
         const int slot = c % kDartSlots;
-        if (!wait_for(&sh.ready[slot], c + 1, nullptr)) {
-            if (lane == 0) sh.failed = 1;
-            return;
-        }
+        if (!wait_for(&sh.ready[slot], c + 1, nullptr)) return false;
         for (int k = (j0 >> 5) + w; 32 * k < j1; k += nw) {
             const int j = 32 * k + lane;
             const bool in = ((sh.bits[slot][k] >> lane) & 1u) && j >= j0 && j < j1;
@@ -786,6 +782,7 @@ __global__ void __launch_bounds__(1024, 1) k_dart_cluster(DevGrid g, DartParams 
             at = __shfl_sync(0xffffffffu, at, 0);
             if (left) sh.queue[queue][at + __popc(m & ((1u << lane) - 1u))] = (uint16_t)j;
         }
+        return true;
     };
     uint64_t n0 = 0;
     uint32_t c = 0;
@@ -804,9 +801,8 @@ __global__ void __launch_bounds__(1024, 1) k_dart_cluster(DevGrid g, DartParams 
         const float root = sqrtf(m2), r = fmaf(root, 1.00001f, prm.cell_slack);
         const float hint_m2 = hint_radius_sq(prm, m2, root);
         if (!tested) {
-            hint_tests(c, (int)(n0 - chunk), (int)(n1 - chunk), hint_m2, queue, warp, 32);
-            __syncthreads();
-            if (sh.failed) break;
+            failed = __syncthreads_or(!hint_tests(c, (int)(n0 - chunk), (int)(n1 - chunk), hint_m2, queue, warp, 32));
+            if (failed) break;
         }
         const auto position = [&](int j, float p[3]) {
 #pragma unroll
@@ -818,6 +814,7 @@ __global__ void __launch_bounds__(1024, 1) k_dart_cluster(DevGrid g, DartParams 
         // same radius: a hint seen early or late is an accepted point
         const bool more = n1 < prm.scatter_count;
         tested = more && n1 != boundary;
+        bool came = true;
         if (warp == 0) {
             walk(sh, acc, link, prm, position, p0, m2);
             if (lane == 0) {
@@ -826,10 +823,10 @@ __global__ void __launch_bounds__(1024, 1) k_dart_cluster(DevGrid g, DartParams 
             }
         } else if (tested) {
             const uint64_t next_end = min(min(n1 + kDartChunk, (uint64_t)prm.scatter_count), boundary);
-            hint_tests(c + 1, 0, (int)(next_end - n1), hint_m2, queue ^ 1, warp - 1, 31);
+            came = hint_tests(c + 1, 0, (int)(next_end - n1), hint_m2, queue ^ 1, warp - 1, 31);
         }
-        __syncthreads();
-        if (sh.done || sh.failed) break;
+        failed = __syncthreads_or(!came);
+        if (failed || sh.done) break;
         if (tested) queue ^= 1;
         n0 = n1;
         if (n1 == chunk_end) {
@@ -842,7 +839,7 @@ __global__ void __launch_bounds__(1024, 1) k_dart_cluster(DevGrid g, DartParams 
     float* dst = out_pts + (size_t)iter * prm.hard_limit * 3;
     for (int k = tid; k < 3 * pc; k += 1024) dst[k] = acc[k];
     if (tid == 0) {
-        out_count[iter] = sh.failed ? -1 : pc;
+        out_count[iter] = failed ? -1 : pc;
         out_last_m2[iter] = sh.last;
     }
     cluster_sync();  // helpers may still write slots

@@ -115,3 +115,21 @@ def test_scatter_points_batch_sizes(gpu_ctx, kw):
             assert np.array_equal(p[i].view(np.uint32), pts[i].view(np.uint32)), (n, i)
     check_iterations(gpu_ctx, sc, opts, 3, 1)
     check_iterations(gpu_ctx, sc, opts, 172, 1)
+
+
+@pytest.mark.parametrize("target", [1, 3, 9, 40, 200])
+def test_early_ends_on_clusters(gpu_ctx, target):
+    """Iterations that end while their helper CTAs are at every stage of the
+    chunks ahead (18 of them): each helper leaves as a whole, and the points are
+    those of one CTA alone."""
+    sc = scenes.small(n_points=16, res=64)
+    scenes.load_into(gpu_ctx, sc)
+    opts = lgm.scatter_opts(scatter_count=60000, target_size=target, hard_limit=target + 2, min_dist_mult=0.2)
+    alone, r2 = gpu_ctx.scatter_points(0, 100, opts)
+    assert max(len(p) for p in alone) == target + 1
+    for _ in range(8):
+        for n in (50, 70):  # clusters of three and of two
+            pts, q = gpu_ctx.scatter_points(0, n, opts)
+            assert np.array_equal(np.asarray(q), np.asarray(r2)[:n], equal_nan=True)
+            for i in range(n):
+                assert np.array_equal(pts[i].view(np.uint32), alone[i].view(np.uint32)), (n, i)
