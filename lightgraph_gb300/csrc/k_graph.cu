@@ -40,6 +40,13 @@ __device__ __forceinline__ bool pair_close(const float* pi, const float* pj, flo
     return e2 < (double)r2;
 }
 
+// A graph's sum of candidate counts from here on: some list does not hold all
+// of its row's partners, which rules the sweep form out. (Set by a maximum, not
+// added: the counts of all other rows together stay below 2^23, so it is neither
+// reached by them nor carried past 2^31.)
+constexpr int32_t kListsOverflow = 1 << 30;
+static_assert(65535 * kCandCap < (1 << 23), "the largest graph with full lists");
+
 // One warp per row; rows of all graphs in one launch.
 __global__ void __launch_bounds__(256) k_candidates(const float* __restrict__ pts,
                                                     const GraphInfo* __restrict__ graphs,
@@ -70,8 +77,10 @@ __global__ void __launch_bounds__(256) k_candidates(const float* __restrict__ pt
     }
     if (lane == 0) {
         cand_cnt[row] = cnt;
-        // (a list that does not hold them all rules the sweep form out)
-        if (sums) atomicAdd(sums + pt_graph[row], cnt > kCandCap ? 1 << 20 : cnt);
+        if (sums) {
+            if (cnt > kCandCap) atomicMax(sums + pt_graph[row], kListsOverflow);
+            else atomicAdd(sums + pt_graph[row], cnt);
+        }
     }
 }
 
@@ -82,7 +91,7 @@ __global__ void __launch_bounds__(256) k_candidates(const float* __restrict__ pt
 // 4096 points with 22 partners 0.51 against 0.13 ms; 3531 points with 160
 // partners 0.44 against 1.3 ms.
 __device__ __forceinline__ bool sweep_form(int n, int32_t sum) {
-    return sum < (1 << 20) && (int64_t)n * (n - 160) > 45 * 2 * (int64_t)sum;
+    return sum < kListsOverflow && (int64_t)n * (n - 160) > 45 * 2 * (int64_t)sum;
 }
 
 // One CTA per graph. Candidate rows are staged into shared memory in chunks
@@ -429,7 +438,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_pair_finish(const GraphInfo*
     if (!sweep_form(n, sums[blockIdx.x])) return;
     if (left >= (1 << 30)) {
         __syncthreads();
-        if (threadIdx.x == 0) sums[blockIdx.x] = 1 << 20;
+        if (threadIdx.x == 0) sums[blockIdx.x] = kListsOverflow;
         return;
     }
     uint32_t* states = ps.states + g.pt_off * kPairStateWords;

@@ -65,3 +65,33 @@ def test_partners_below_overflow(gpu_ctx, near):
         for g, (c, c2) in enumerate([(p, r2), (q, q2)]):
             ref, ne_ref = po.build_graph(c, c2, cap)
             assert np.array_equal(adj[g], ref) and ne[g] == ne_ref
+
+
+def lattice_ball(n, partners):
+    """A jittered lattice in a ball, in order of the distance from its centre."""
+    rng = np.random.default_rng(2)
+    m = np.arange(-14, 15)
+    g = np.stack(np.meshgrid(m, m, m, indexing="ij"), -1).reshape(-1, 3) + rng.uniform(-0.2, 0.2, (29 ** 3, 3))
+    near = np.argsort(np.linalg.norm(g, axis=1))[:n]
+    return (g[near] * 0.05).astype(np.float32), np.float32(0.05 * (partners * 0.75 / np.pi) ** (1.0 / 3.0))
+
+
+@pytest.mark.parametrize("n, partners, lists, below", [
+    (4700, 200.0, (2048, 4700), (0, 96)),   # past 2047 lists overflow, and no list of partners below does
+    (4700, 188.0, (1024, 2047), (0, 96)),
+    (4096, 900.0, (2048, 4096), (97, 4096)),  # dense throughout
+])
+def test_many_lists_overflow(gpu_ctx, n, partners, lists, below):
+    """Graphs in which more rows have more than 96 partners past them than a
+    32-bit sum of 2^20 each could count."""
+    from scipy.spatial import cKDTree
+    p, r = lattice_ball(n, partners)
+    pairs = cKDTree(p.astype(np.float64)).query_pairs(float(r), output_type="ndarray")
+    over = (np.bincount(pairs.min(axis=1), minlength=n) > 96).sum()
+    assert lists[0] <= over <= lists[1]
+    assert below[0] <= np.bincount(pairs.max(axis=1), minlength=n).max() <= below[1]
+    r2 = r * r
+    for cap in (12, 100, 255):
+        adj, ne = gpu_ctx.build_graphs([p], [r2], cap, want_adjacency=True)
+        ref, ne_ref = po.build_graph(p, r2, cap)
+        assert np.array_equal(adj[0], ref) and ne[0] == ne_ref, cap
