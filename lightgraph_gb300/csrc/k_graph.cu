@@ -425,7 +425,9 @@ static_assert(2 * kWords + 1 <= kPairStateWords && 2 * kWords < 32, "a state is 
 
 // One CTA per graph: passes over the points that the sweeps left undecided, if
 // any, then the edges (i, j), i < j, in order. A graph whose lists overflow is
-// left to k_greedy (sums[graph] says so).
+// left to k_greedy (sums[graph] says so). So is one in which a pass decides
+// nothing, which complete lists rule out: there are no more passes than pairs,
+// whatever the lists hold.
 __global__ void __launch_bounds__(kFinishThreads) k_pair_finish(const GraphInfo* __restrict__ graphs,
                                                                 const uint16_t* __restrict__ cand,
                                                                 const int32_t* __restrict__ cand_cnt, int max_connect,
@@ -445,7 +447,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_pair_finish(const GraphInfo*
     if (left) {
         const uint32_t lt = (1u << lane) - 1u;
         for (;;) {
-            bool open = false;
+            bool open = false, decided = false;
             for (int v = warp; v < n; v += kFinishThreads / 32) {
                 uint32_t* st = states + (size_t)v * kPairStateWords;
                 if (!__any_sync(0xffffffffu, lane < kWords && st[kWords + lane] != 0u)) continue;
@@ -460,10 +462,17 @@ __global__ void __launch_bounds__(kFinishThreads) k_pair_finish(const GraphInfo*
                 }
                 x.limit = ld_limit(ps.limits + row);
                 __syncwarp();
-                if (pair_decide(x, v, max_connect, lt, ps.limits + g.pt_off)) pair_store(x, st, lane);
+                if (pair_decide(x, v, max_connect, lt, ps.limits + g.pt_off)) {
+                    pair_store(x, st, lane);
+                    decided = true;
+                }
                 open |= __any_sync(0xffffffffu, x.und != 0u);
             }
             if (!__syncthreads_or(open)) break;
+            if (!__syncthreads_or(decided)) {
+                if (threadIdx.x == 0) sums[blockIdx.x] = kListsOverflow;
+                return;
+            }
         }
     }
     int2* E = edges + g.e_off;
