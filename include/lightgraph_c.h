@@ -364,9 +364,9 @@ uint64_t lg_frame_launches(const lg_ctx* ctx);
 
 /* Schedule of the path solve over all loaded graphs. -1 (default): a single
  * graph, a few small ones (up to eight of together 4096 points) and batches with
- * large ones are solved from their edges, up to 9200 points a graph and 16 edges
- * a point (a distance is the sum along a shortest path, rounded to FP32 once,
- * and infinity where its squared transmittance underflows in FP64); others by
+ * large ones are solved from their edges, up to 8928 points a graph and 16 edges
+ * a point, as long as no edge can be over 2^20 times as deep as another (a
+ * distance is the sum along a shortest path, rounded to FP32 once); others by
  * Floyd-Warshall on the schedule chosen by the autotuner, which times every
  * candidate once per (graph count, largest graph) on a scratch copy and keeps
  * the fastest; 0: two launches per round per graph; 1 or 2: one persistent

@@ -16,26 +16,32 @@
 // same in any, since a distance only ever falls and its least is the least
 // over all paths.
 //
-// The passes count distances in 32-bit integers, which makes every sum exact
-// and every edge at least one unit long: the paths they settle on are trees.
-// What the edges of a path lost by being rounded to units, kept in fractions of
-// a unit, is then summed down the trees, and the distance handed out is rounded
-// to FP32 once. Relative to FP64 the benchmark graphs' distances are off by
-// 2.5e-8 to 2.6e-8 here and 3.9e-8 to 4.5e-8 with Floyd-Warshall (root mean square).
-// 2^32 units reach a depth at which the reference's own comparison of squared
-// transmittances underflows in FP64 (Ctx::path_unit): beyond it there is no path
-// there either. Of paths that agree to within a unit or so either may be taken.
+// The passes add in FP32, rounded up: a distance never falls short of the one it
+// came from, so the edges by which the distances came form trees (an edge of
+// depth 0 counts as the least number above it). What each edge of a path was
+// rounded by, an exact difference, is then summed down the trees in 64-bit
+// integers, and the sum of distance and correction is rounded to FP32 once. What
+// is left of the rounding is in the choice between paths that nearly tie, by
+// less than Floyd-Warshall's own sums as long as a graph's depths lie within a
+// factor of 2^20 of one another (Ctx::depths_near). Against FP64, 4096 random points,
+// density uniform / over a range of 10^4: root mean square 2.5e-8 / 2.6e-8, largest
+// 6.0e-8 / 2.2e-7; Floyd-Warshall 4.4e-8 / 4.7e-8 and 2.3e-7 / 2.5e-7. The same in
+// thin volumes as in thick ones, and finite wherever there is a path. Of paths of
+// the same rounded length the one through the lowest place is taken.
 //
 // LightGraph's edges are symmetric and non-negative, and few; dense or
 // directed matrices are solved by k_fw.cu.
 //
 // Bound by shared-memory loads, 16 bytes for four sums in rows of 4 K bytes that
 // meet in the same banks 1.5 (K = 16) to ~2.6 times (K = 4), and by the barriers
-// of the passes where a graph is small; summing the lost fractions takes a
-// sixth of the time. Against the symmetric Floyd-Warshall with its fill and
-// mirror, preparation and mirror included: 200 points 0.051 against 0.10 ms, 1024
-// points 0.15 against 0.37 ms, 2500 points 0.74 against 0.93 ms, 4096 points 2.04
-// against 2.53 ms, 8 graphs of 4096 points 11.0 against 19.7 ms.
+// of the passes where a graph is small; summing the corrections takes a
+// fifth of the time. March, preparation and mirror included, against march, fill
+// and the symmetric Floyd-Warshall: 200 points 0.072 against 0.130 ms, 1024 points
+// 0.17 against 0.39 ms, 2500 points 0.71 against 0.99 ms, 4096 points 1.70 against
+// 2.55 ms, 8900 points 9.6 against 24.4 ms, 24 graphs of 2500 points 10.9 against
+// 15.2 ms. (Distances as integers of one unit of optical depth for all graphs, with
+// corrections of 18 bits: 4096 points 1.65 ms, 24 of 2500 10.3 ms; but the unit was
+// coarser than FP32 in thin volumes, where paths were off by up to 1%.)
 #include <algorithm>
 
 #include "lg_kernels.h"
@@ -53,44 +59,34 @@ __device__ __forceinline__ uint32_t spread_bits4(uint32_t v) {
     return (v | (v << 2)) & 0x249u;
 }
 
+constexpr uint32_t kFar = 0x7F800000u;  // the bits of inf: no path
+
+// A word per vertex and source: the place that the vertex's path leads through,
+// and the correction from there.
+constexpr int kSumBits = 50;
+constexpr unsigned long long kSumMask = (1ull << kSumBits) - 1;
+__device__ __forceinline__ unsigned long long path_word(uint32_t place, long long sum) {
+    return ((unsigned long long)place << kSumBits) | ((unsigned long long)sum & kSumMask);
+}
+
 // One CTA per graph: numbers the vertices along a Morton curve over their
 // bounding box (perm: place -> vertex, rank: vertex -> place; by vertex inside
 // a cell) and lays the edges out in pairs, edge pair p of place v at
 // ell[p * n + v] as {neighbour's place, depth, neighbour's place, depth};
-// unused halves repeat the first edge. The neighbour is a place, the depth in
-// units; rest holds, at the same places, path_word of the neighbour and what the
-// depth is off by. step: a fifth of the mean depth. The order of a vertex's
-// edges is left to chance and does not reach the distances.
-// A word per vertex and source: the place that the vertex's path leads through,
-// and what the units from there are off by, in fractions that (n - 1) edges
-// each off by a whole unit cannot overflow.
-__device__ __forceinline__ uint32_t path_word(int place, int rest) { return ((uint32_t)place << 18) | ((uint32_t)rest & 0x3FFFFu); }
-__device__ __forceinline__ int path_fraction_bits(int n) { return min(10, 17 - (32 - __clz(n - 1))); }
-
-// Depth w in 2^-bits units, to the nearest: w's 24 bits times the 64 of pu.per.
-// Integers, since FP64 runs at 1/64 of their rate (with it here and where the
-// distances are handed out, 32 graphs of 257 to 3805 points took 8.00 ms, not 7.76).
-__device__ __forceinline__ uint64_t path_units(const PathUnit& pu, float w, int bits) {
-    const uint32_t b = __float_as_uint(w) & 0x7FFFFFFFu;
-    const int e = max((int)(b >> 23), 1);
-    const uint64_t m = (b & 0x7FFFFFu) | (b >> 23 ? 0x800000u : 0u);
-    const uint64_t v = m * (uint32_t)(pu.per >> 32) + ((m * (uint32_t)pu.per) >> 32);
-    const int s = 182 - e - pu.exponent - bits;  // at least 12: the result stays below 2^43
-    return s > 63 ? 0 : (v + (1ull << (s - 1))) >> s;
-}
-
+// unused halves repeat the first edge. The depth is the bits of a float, the
+// least one for an edge of depth 0. step: a fifth of the mean depth. The order
+// of a vertex's edges is left to chance and does not reach the distances.
 __global__ void __launch_bounds__(kPrepThreads) k_path_prep(const float* __restrict__ pts,
                                                             const GraphInfo* __restrict__ graphs,
                                                             const int2* __restrict__ edges,
                                                             const int32_t* __restrict__ edge_cnt,
-                                                            const float* __restrict__ W, PathUnit pu, int stride,
+                                                            const float* __restrict__ W, int stride,
                                                             uint16_t* __restrict__ perm, uint16_t* __restrict__ rank,
-                                                            int4* __restrict__ ell, uint32_t* __restrict__ rest,
-                                                            uint32_t* __restrict__ step) {
+                                                            int4* __restrict__ ell, float* __restrict__ step) {
     extern __shared__ __align__(16) int prep_shared[];  // cell offsets, then a degree, a place and a cell member per vertex
     __shared__ float red[6][32];
     __shared__ int warp_sum[32];
-    __shared__ unsigned long long total;
+    __shared__ float total;
     __shared__ int finite;
     const GraphInfo g = graphs[blockIdx.x];
     const int n = g.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -111,7 +107,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_path_prep(const float* __restr
     }
     for (int i = tid; i < kCells; i += kPrepThreads) cell[i] = 0;
     if (tid == 0) {
-        total = 0;
+        total = 0.f;
         finite = 0;
     }
 #pragma unroll
@@ -173,10 +169,8 @@ __global__ void __launch_bounds__(kPrepThreads) k_path_prep(const float* __restr
     }
     __syncthreads();
     int2* row = reinterpret_cast<int2*>(ell) + g.pt_off * stride;
-    uint32_t* off = rest + g.pt_off * stride;
     const int ne = edge_cnt[blockIdx.x];
-    const int bits = path_fraction_bits(n);
-    unsigned long long sum = 0;
+    float sum = 0.f;
     int cnt = 0;
     for (int e0 = tid; e0 < ne; e0 += 4 * kPrepThreads) {
         float ws[4];
@@ -189,18 +183,13 @@ __global__ void __launch_bounds__(kPrepThreads) k_path_prep(const float* __restr
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            if (!(ws[k] <= pu.longest)) continue;  // dropped, or past the last depth that matters
-            const uint64_t units = path_units(pu, ws[k], bits);
-            const int d = (int)max(1u, (uint32_t)((units + ((1ull << bits) >> 1)) >> bits));
-            const int lost = (int)((int64_t)units - ((int64_t)(uint32_t)d << bits));
+            if (!(ws[k] < kInf)) continue;  // dropped
+            const int d = max(__float_as_int(ws[k]), 1);
             const int a = place[es[k].x], b = place[es[k].y];
             const int ka = atomicAdd(deg + a, 1), kb = atomicAdd(deg + b, 1);
-            const int64_t ia = ((int64_t)(ka >> 1) * n + a) * 2 + (ka & 1), ib = ((int64_t)(kb >> 1) * n + b) * 2 + (kb & 1);
-            row[ia] = make_int2(b, d);
-            row[ib] = make_int2(a, d);
-            off[ia] = path_word(b, lost);
-            off[ib] = path_word(a, lost);
-            sum += (unsigned)d;
+            row[((int64_t)(ka >> 1) * n + a) * 2 + (ka & 1)] = make_int2(b, d);
+            row[((int64_t)(kb >> 1) * n + b) * 2 + (kb & 1)] = make_int2(a, d);
+            sum += ws[k];
             ++cnt;
         }
     }
@@ -216,18 +205,22 @@ __global__ void __launch_bounds__(kPrepThreads) k_path_prep(const float* __restr
         const int2 any = deg[i] > 0 ? row[(int64_t)i * 2] : make_int2(i, 1);
         for (int k = deg[i]; k < stride; ++k) row[((int64_t)(k >> 1) * n + i) * 2 + (k & 1)] = any;
     }
-    if (tid == 0) step[blockIdx.x] = (uint32_t)max(1ull, finite > 0 ? total / (unsigned)finite / 5u : 1ull);
+    // (the sum's last bits, and so the passes, are left to chance too)
+    if (tid == 0) step[blockIdx.x] = finite > 0 ? total / (5.f * (float)finite) : 0.f;
 }
 
 // Shared memory of a k_paths CTA for n vertices: the distances, then pending
-// values, marks and two lists, or in their place four bits a distance and a
-// word per vertex.
+// values, marks and two lists (9 bytes a vertex), or in their place four bits a
+// distance and a word per vertex.
 __host__ __device__ constexpr size_t path_smem(int n, int K) {
     const size_t n16 = ((size_t)n + 15) / 16 * 16;
-    return (size_t)n * 4 * K + n16 * (K / 2 + 4 > 9 ? K / 2 + 4 : 9);
+    return (size_t)n * 4 * K + n16 * (K / 2 + 8);
 }
 
-__device__ __forceinline__ uint32_t add_min(uint32_t x, uint32_t w, uint32_t m) { return __viaddmin_u32(x, w, m); }
+// Distances are the bits of floats from 0 to inf, which compare as integers.
+__device__ __forceinline__ uint32_t add_up(uint32_t x, int w) {
+    return __float_as_uint(__fadd_ru(__uint_as_float(x), __int_as_float(w)));
+}
 
 // Room for the warp's c values each in a list of *count: where the lane's begin.
 __device__ __forceinline__ int claim(int* count, int c, int lane) {
@@ -249,11 +242,10 @@ __device__ __forceinline__ uint4 relax(const uint4* d, const int4* __restrict__ 
                                        uint4 m) {
     auto pair = [&](int4 r) {
         const uint4 x = d[r.x * Q + q], y = d[r.z * Q + q];
-        const uint32_t a = (uint32_t)r.y, b = (uint32_t)r.w;
-        m.x = add_min(y.x, b, add_min(x.x, a, m.x));
-        m.y = add_min(y.y, b, add_min(x.y, a, m.y));
-        m.z = add_min(y.z, b, add_min(x.z, a, m.z));
-        m.w = add_min(y.w, b, add_min(x.w, a, m.w));
+        m.x = __vimin3_u32(m.x, add_up(x.x, r.y), add_up(y.x, r.w));
+        m.y = __vimin3_u32(m.y, add_up(x.y, r.y), add_up(y.y, r.w));
+        m.z = __vimin3_u32(m.z, add_up(x.z, r.y), add_up(y.z, r.w));
+        m.w = __vimin3_u32(m.w, add_up(x.w, r.y), add_up(y.w, r.w));
     };
     if constexpr (kPairs > 0) {
         int4 r[kPairs];
@@ -274,18 +266,17 @@ __device__ __forceinline__ uint4 relax(const uint4* d, const int4* __restrict__ 
 template <int Q, int kPairs>
 __global__ void __launch_bounds__(1024) k_paths(const GraphInfo* __restrict__ graphs, const uint16_t* __restrict__ perm,
                                                 const uint16_t* __restrict__ rank, const int4* __restrict__ ell,
-                                                const uint32_t* __restrict__ rest,
-                                                const uint32_t* __restrict__ steps, int half, PathUnit pu, int n_min,
-                                                int n_max, float* __restrict__ S) {
+                                                const float* __restrict__ steps, int half, int n_min, int n_max,
+                                                float* __restrict__ S) {
     constexpr int K = 4 * Q;
     extern __shared__ __align__(16) uint8_t path_shared[];
     __shared__ int count[2], going[2];
-    __shared__ uint32_t low[2];
+    __shared__ uint32_t low[2], top;
     const GraphInfo g = graphs[blockIdx.y];
     const int n = g.n, tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
     const int s0 = blockIdx.x * K;
     if (s0 >= n || n <= n_min || n > n_max) return;
-    const uint32_t far = pu.far;
+    constexpr uint32_t far = kFar;
     const int n16 = (n + 15) / 16;
     uint4* d = reinterpret_cast<uint4*>(path_shared);
     uint32_t* pending = reinterpret_cast<uint32_t*>(d + (size_t)Q * n);  // least distance not passed on yet
@@ -294,7 +285,7 @@ __global__ void __launch_bounds__(1024) k_paths(const GraphInfo* __restrict__ gr
     uint16_t* go = list + 16 * n16;
     const int4* edge = ell + g.pt_off * half;
     const int ns = min(K, n - s0);
-    const uint32_t step = steps[blockIdx.y];
+    const float step = steps[blockIdx.y];
     for (int i = tid; i < Q * n; i += nt) d[i] = make_uint4(far, far, far, far);
     for (int i = tid; i < 16 * n16; i += nt) pending[i] = i >= s0 && i < s0 + ns ? 0u : far;
     for (int i = tid; i < n16; i += nt) reinterpret_cast<uint4*>(mark)[i] = make_uint4(0, 0, 0, 0);
@@ -302,10 +293,11 @@ __global__ void __launch_bounds__(1024) k_paths(const GraphInfo* __restrict__ gr
         count[tid] = 0;
         going[tid] = 0;
         low[tid] = far;
+        top = 0u;
     }
     __syncthreads();
     if (tid < ns) reinterpret_cast<uint32_t*>(d)[(s0 + tid) * K + tid] = 0u;
-    uint32_t bound = min(step, far - 1u);
+    uint32_t bound = min(__float_as_uint(step), far - 1u);
     const bool small = n <= 4 * nt;
     for (int par = 0;; par ^= 1) {
         // 1. the vertices whose distances fell to the bound or below, and the
@@ -393,25 +385,25 @@ __global__ void __launch_bounds__(1024) k_paths(const GraphInfo* __restrict__ gr
         // (200 points: 0.070 -> 0.055 ms, of them chains of few neighbours 0.19 ->
         // 0.07 ms; 4096 points: 2.23 -> 2.36 ms, so not in a large one). It stays
         // below far, the mark of vertices with nothing pending.
-        const uint32_t by = small && items > 0 ? (uint32_t)min(max(nt / items, 1), 4) : 1u;
-        const uint32_t room = far - 1u - bound;
-        bound = items == 0 ? waiting : room / by > step ? bound + by * step : far - 1u;
+        const float by = small && items > 0 ? (float)min(max(nt / items, 1), 4) : 1.f;
+        bound = items == 0 ? waiting : min(__float_as_uint(fmaf(by, step, __uint_as_float(bound))), far - 1u);
         __syncthreads();
     }
     // The edge by which each distance came: of those that give it, the one to
     // the lowest place. Four bits each; d tells where there is none.
     uint16_t* by = reinterpret_cast<uint16_t*>(d + (size_t)Q * n);
+    uint32_t most = 0;
     for (int i = tid; i < Q * n; i += nt) {
         const int v = i / Q, q = i % Q;
         const uint4 m = d[i];
         uint32_t best[4] = {~0u, ~0u, ~0u, ~0u};  // place, edge
-        auto tie = [&](uint32_t u, uint32_t w, uint32_t slot) {
+        auto tie = [&](uint32_t u, int w, uint32_t slot) {
             const uint4 x = d[u * Q + q];
             const uint32_t key = (u << 4) | slot;
-            if (x.x + w == m.x) best[0] = min(best[0], key);
-            if (x.y + w == m.y) best[1] = min(best[1], key);
-            if (x.z + w == m.z) best[2] = min(best[2], key);
-            if (x.w + w == m.w) best[3] = min(best[3], key);
+            if (add_up(x.x, w) == m.x) best[0] = min(best[0], key);
+            if (add_up(x.y, w) == m.y) best[1] = min(best[1], key);
+            if (add_up(x.z, w) == m.z) best[2] = min(best[2], key);
+            if (add_up(x.w, w) == m.w) best[3] = min(best[3], key);
         };
 #pragma unroll 3
         for (int k = 0; k < half; ++k) {
@@ -420,35 +412,48 @@ __global__ void __launch_bounds__(1024) k_paths(const GraphInfo* __restrict__ gr
             tie(r.z, r.w, 2 * k + 1);
         }
         by[i] = (uint16_t)((best[0] & 15u) | ((best[1] & 15u) << 4) | ((best[2] & 15u) << 8) | ((best[3] & 15u) << 12));
+        const uint32_t ms[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) most = max(most, ms[c] < far ? ms[c] : 0u);
     }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0) atomicMax(&top, most);
     __syncthreads();
     // Source by source: each vertex's word starts as its edge's and takes over
     // the word of the place it names until that is the source. Words only move
     // towards the source and their sums are exact, so another's may be read at
-    // any stage. Then the source's row of the matrix, columns in vertex
-    // order; the padding is inf.
-    volatile uint32_t* word = reinterpret_cast<uint32_t*>(by + (size_t)Q * n + (Q * n & 1));
+    // any stage (8 bytes are read and written at once). Then the source's row of
+    // the matrix, columns in vertex order; the padding is inf.
+    volatile unsigned long long* word =
+        reinterpret_cast<volatile unsigned long long*>(by + ((size_t)Q * n + 3) / 4 * 4);
     const uint16_t* rk = rank + g.pt_off;
-    const uint32_t* off = rest + g.pt_off * 2 * half;
+    const int2* lone = reinterpret_cast<const int2*>(edge);
     const uint32_t* dist = reinterpret_cast<const uint32_t*>(d);
-    // a distance of x = a 2^20 + b fractions in FP32, as c1 a + c0 b with the
-    // factors' second halves: off by little more than the one rounding
-    const int bits = path_fraction_bits(n);
-    const double scale = 1.0 / ((double)(1 << bits) * pu.per_unit);
-    const float c0 = (float)scale, c0_lo = (float)(scale - (double)c0);
-    const float c1 = (float)(scale * 1048576.0), c1_lo = (float)(scale * 1048576.0 - (double)c1);
+    // Rounding up adds less than a unit in the last place of the CTA's largest
+    // distance to an edge (one such unit where the depth is 0): 2^(49 - log2 n)
+    // fractions to that unit. A power of two in two factors, since it can exceed a float's.
+    const int fine = 23 - ((int)(top >> 23) - 127) + kSumBits - 1 - (32 - __clz(n - 1));
+    auto power = [](int e) { return __int_as_float((e + 127) << 23); };
+    const int fine0 = min(fine, 100);
+    const float up0 = power(fine0), up1 = power(fine - fine0), down0 = power(-fine0), down1 = power(fine0 - fine);
     float* M = S + g.s_off;
     for (int k = 0; k < ns; ++k) {
         const int root = s0 + k;
         for (int v0 = tid; v0 < n; v0 += 4 * nt) {
-            uint32_t w[4];
+            unsigned long long w[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int v = v0 + c * nt;
                 w[c] = path_word(root, 0);
                 if (v >= n || v == root || dist[v * K + k] >= far) continue;
                 const uint32_t slot = (by[v * Q + k / 4] >> (4 * (k & 3))) & 15u;
-                w[c] = __ldg(off + ((int64_t)(slot >> 1) * n + v) * 2 + (slot & 1u));
+                const int2 r = __ldg(lone + ((int64_t)(slot >> 1) * n + v) * 2 + (slot & 1u));
+                // (dist[r.x] + depth) - dist[v], exact but for bits far below the fractions
+                const float x = __uint_as_float(dist[r.x * K + k]), y = r.y == 1 ? 0.f : __int_as_float(r.y);
+                const float s = __fadd_rn(x, y), b = __fsub_rn(s, x);
+                const float err = __fadd_rn(__fsub_rn(x, __fsub_rn(s, b)), __fsub_rn(y, b));
+                const float lost = __fadd_rn(err, __fsub_rn(s, __uint_as_float(dist[v * K + k])));
+                w[c] = path_word((uint32_t)r.x, __float2ll_rn(lost * up0 * up1));
             }
 #pragma unroll
             for (int c = 0; c < 4; ++c)
@@ -458,16 +463,16 @@ __global__ void __launch_bounds__(1024) k_paths(const GraphInfo* __restrict__ gr
         for (bool more = true; more;) {  // all of a thread's vertices a step at a time: log2(path) steps
             more = false;
             for (int v0 = tid; v0 < n; v0 += 4 * nt) {
-                uint32_t w[4], u[4];
+                unsigned long long w[4], u[4];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) w[c] = v0 + c * nt < n ? word[v0 + c * nt] : path_word(root, 0);
 #pragma unroll
-                for (int c = 0; c < 4; ++c) u[c] = word[w[c] >> 18];
+                for (int c = 0; c < 4; ++c) u[c] = word[w[c] >> kSumBits];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    if ((int)(w[c] >> 18) == root) continue;
-                    word[v0 + c * nt] = (u[c] & ~0x3FFFFu) | ((w[c] + u[c]) & 0x3FFFFu);
-                    more |= (int)(u[c] >> 18) != root;
+                    if ((int)(w[c] >> kSumBits) == root) continue;
+                    word[v0 + c * nt] = (u[c] & ~kSumMask) | ((w[c] + u[c]) & kSumMask);
+                    more |= (int)(u[c] >> kSumBits) != root;
                 }
             }
         }
@@ -477,12 +482,11 @@ __global__ void __launch_bounds__(1024) k_paths(const GraphInfo* __restrict__ gr
             float out = kInf;
             if (j < n) {
                 const int v = rk[j];
-                const uint32_t m = dist[v * K + k], w = word[v];
-                if (m < far) {
-                    const int64_t x = ((int64_t)m << bits) + ((int)(w << 14) >> 14);
-                    const float a = (float)(uint32_t)(x >> 20), b = (float)(uint32_t)(x & 0xFFFFF);
-                    out = __fmaf_rn(a, c1, __fmaf_rn(b, c0, __fmaf_rn(a, c1_lo, __fmul_rn(b, c0_lo))));
-                }
+                const uint32_t m = dist[v * K + k];
+                const long long sum = (long long)(word[v] << (64 - kSumBits)) >> (64 - kSumBits);
+                // (a path of n edges of depth 0 counts fewer than 2^14 least numbers)
+                if (m < 1u << 14) out = 0.f;
+                else if (m < far) out = __fadd_rn(__uint_as_float(m), __ll2float_rn(sum) * down0 * down1);
             }
             row[j] = out;
         }
@@ -528,14 +532,14 @@ __global__ void k_edge_depths(const GraphInfo* __restrict__ graphs, const int2* 
 int path_stride(int max_connect) { return std::max(2, (max_connect + 1) / 2 * 2); }
 
 cudaError_t launch_paths(const float* pts, const GraphInfo* graphs, int n_graphs, int min_n, int max_n, int64_t n_points,
-                         int max_connect, const int2* edges, const int32_t* edge_cnt, const float* W, const PathUnit& pu,
+                         int max_connect, const int2* edges, const int32_t* edge_cnt, const float* W,
                          const PathScratch& ps, float* S, int sms, cudaStream_t st) {
     if (n_graphs == 0 || max_n == 0) return cudaSuccess;
     const int stride = path_stride(max_connect), half = stride / 2;
     cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k_path_prep));
     if (e != cudaSuccess) return e;
     k_path_prep<<<n_graphs, kPrepThreads, sizeof(int) * (kCells + (size_t)max_n) + 2 * sizeof(uint16_t) * (size_t)max_n, st>>>(
-        pts, graphs, edges, edge_cnt, W, pu, stride, ps.perm, ps.rank, ps.ell, ps.rest, ps.step);
+        pts, graphs, edges, edge_cnt, W, stride, ps.perm, ps.rank, ps.ell, ps.step);
     ++g_launch_counter;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // Sources per CTA: few while that makes CTAs for idle SMs (1024 points: K =
@@ -548,8 +552,9 @@ cudaError_t launch_paths(const float* pts, const GraphInfo* graphs, int n_graphs
     const int64_t groups = (n_points + 15) / 16;
     if (n_points <= 11 * (int64_t)sms) Q = 1;
     else if (groups > sms && groups < 2 * (int64_t)sms) Q = 2;
-    constexpr int n_max4 = 3040, n_max2 = 5640, kSmall = 1700;
+    constexpr int n_max4 = 2896, n_max2 = 5280, kSmall = 1700;
     constexpr size_t most = 227 * 1024 - 64;  // less the static words
+    static_assert(kPathMaxPoints <= 1 << 14, "places in the words");
     static_assert(path_smem(n_max4, 16) <= most && path_smem(n_max2, 8) <= most && path_smem(kPathMaxPoints, 4) <= most);
     auto run = [&](auto pairs6, auto pairs, int K, int n_min, int n_max) {
         n_max = std::min(n_max, max_n);
@@ -557,7 +562,7 @@ cudaError_t launch_paths(const float* pts, const GraphInfo* graphs, int n_graphs
         auto kernel = half == 6 ? pairs6 : pairs;
         if ((e = raise_smem_limit(reinterpret_cast<const void*>(kernel))) != cudaSuccess) return;
         kernel<<<dim3((n_max + K - 1) / K, n_graphs), n_max > kSmall ? 512 : 256, path_smem(n_max, K), st>>>(
-            graphs, ps.perm, ps.rank, ps.ell, ps.rest, ps.step, half, pu, n_min, n_max, S);
+            graphs, ps.perm, ps.rank, ps.ell, ps.step, half, n_min, n_max, S);
         ++g_launch_counter;
         e = cudaGetLastError();
     };

@@ -947,32 +947,49 @@ lg_status Ctx::march_edges() {
     CK(launch_fill(d_S.as<float>(), s_floats, INFINITY, st), "S fill");
     CK(launch_edge_march(scene(), d_pts.as<float>(), d_graphs.as<GraphInfo>(), n_graphs, max_edges,
                          d_edges.as<int2>(), d_edge_cnt.as<int32_t>(), d_S.as<float>(), nullptr, st), "edge march");
-    marched = {true, {shader.extinction[0], shader.extinction[1], shader.extinction[2], settings.cutoff}};
+    marched = {true, depths_near(), {shader.extinction[0], shader.extinction[1], shader.extinction[2], settings.cutoff}};
     return LG_OK;
 }
 
 bool Ctx::marched_as_set() const {
-    return marched.valid && marched.by[0] == shader.extinction[0] && marched.by[1] == shader.extinction[1] &&
-           marched.by[2] == shader.extinction[2] && marched.by[3] == settings.cutoff;
+    return marched.valid && marched.near && marched.by[0] == shader.extinction[0] &&
+           marched.by[1] == shader.extinction[1] && marched.by[2] == shader.extinction[2] &&
+           marched.by[3] == settings.cutoff;
 }
 
-// Whether the paths are solved from the edges (k_paths.cu), and in which unit: as
-// fine as lets 32 bits hold a depth R at which the squared transmittance of
-// every channel underflows in FP64 (2 a R > 745), where the reference's
-// comparison of squared lengths sees no path, plus one edge.
+// Whether the depths of edges marched under the settings are non-negative and
+// close enough to one another for k_paths: a sample that counts adds a step of
+// at least the cutoff or the least density and of at most the greatest, and an
+// edge past the dropout depth is none. (A negative cutoff lets negative depths
+// through. With the default shader and a radius of 30 voxels they lie within
+// 2^17, whatever drops out.)
+bool Ctx::depths_near() const {
+    if (!(settings.cutoff >= 0.0) || !D().valid) return false;
+    double a[3];
+    for (int c = 0; c < 3; ++c) a[c] = -shader.extinction[c];
+    float r2 = 0.f;
+    for (const GraphInfo& g : h_graphs) r2 = std::max(r2, g.r2);
+    const double step = settings.step[1];
+    const double least = std::max(settings.cutoff, shader.scatter_density_min) * step;
+    const double longest = std::sqrt((double)r2) / D().g.h + 2.0 * step;
+    const double most = std::min((double)dropout_depth(a, settings.cutoff),
+                                 std::max(shader.density_max, shader.scatter_density_min) * longest);
+    return most > 0.0 && most < 1e30 && least > 1e-30 && most <= kPathDepthRange * least;
+}
+
+// Whether the paths are solved from the edges (k_paths.cu).
 // Floyd-Warshall solves the graphs where a schedule is pinned, a graph is too
-// large for shared memory or has too many edges, depths could be negative (only
-// a negative cutoff lets them through), a channel does not absorb, and in
+// large for shared memory or has too many edges, the depths are not near, and in
 // batches that fill the GPU with it: it takes 0.38 us a point of the largest
 // graph or, if that is more, 1 ms for 2.6e10 (i, j, k); the solve from the edges
 // 1 ms for 1.2e7 (i, j) (16 of 500 points: 0.21 against 0.30 ms, 48 of 750: 1.09
-// against 1.53, 4 of 1500: 0.70 against 0.81, but 8 of 2500: 5.2 against 3.8, 8
-// of 4096: 19.7 against 11.0); up to 2048 points a graph that is hardly ever
-// less, and they are left to the autotuner.
-// Few and small ones leave both at their latency, which is shorter from the edges (8 of 200
-// points: 0.12 against 0.075 ms, 4 of 1000: 0.40 against 0.35).
-bool Ctx::path_unit(PathUnit& pu) const {
-    if (fw_pinned >= 0 || settings.cutoff < 0.0 || max_n > kPathMaxPoints || max_connect > 16) return false;
+// against 1.53, but 8 of 2500: 5.2 against 3.8, 8 of 4096: 19.7 against 11.1); up
+// to 2048 points a graph that is hardly ever less, and they are left to the
+// autotuner. Few and small ones leave both at their latency, which is shorter
+// from the edges (8 of 200 points: 0.14 against 0.09 ms, 4 of 1000: 0.41 against
+// 0.36, 4 of 1500: 0.72 either way).
+bool Ctx::by_edges() const {
+    if (fw_pinned >= 0 || max_n > kPathMaxPoints || max_connect > 16) return false;
     const bool few = n_graphs == 1 || (n_graphs <= 8 && n_points <= 4096);
     if (!few && max_n <= 2048) return false;
     if (!few) {
@@ -983,21 +1000,6 @@ bool Ctx::path_unit(PathUnit& pu) const {
         }
         if (pairs / 1.2e7 >= std::max(3.8e-4 * max_n, triples / 2.6e10)) return false;
     }
-    double a[3], lo = INFINITY, hi = 0.0;
-    for (int c = 0; c < 3; ++c) {
-        a[c] = -shader.extinction[c];
-        lo = std::min(lo, a[c]);
-        hi = std::max(hi, a[c]);
-    }
-    if (!(lo > 1e-30) || !(hi < 1e30) || hi > 4.0 * lo) return false;
-    const double R = 373.0 / lo;
-    // an edge that did not drop out is no deeper than the dropout depth
-    const double edge = std::min(R, 1.0001 * (double)std::max(dropout_depth(a, settings.cutoff), 0.f));
-    if (!(edge > 0.0)) return false;  // every edge drops out
-    pu.per_unit = 4294960000.0 / (R + edge);
-    pu.per = (uint64_t)std::ldexp(std::frexp(pu.per_unit, &pu.exponent), 64);
-    pu.longest = (float)edge;
-    pu.far = (uint32_t)(R * pu.per_unit);
     return true;
 }
 
@@ -1013,22 +1015,22 @@ lg_status Ctx::march_to_edges() {
     return LG_OK;
 }
 
-lg_status Ctx::solve_from_edges(const PathUnit& pu) {
+lg_status Ctx::solve_from_edges() {
     Ctx* ctx = this;
     marched.valid = false;
     const int64_t P = std::max<int64_t>(n_points, 1);
     CK(d_path_order.reserve(2 * sizeof(uint16_t) * P), "path order alloc");
     const size_t places = (size_t)P * path_stride(max_connect);
-    CK(d_path_ell.reserve((sizeof(int2) + sizeof(uint32_t)) * places), "path edges alloc");
-    CK(d_path_step.reserve(sizeof(uint32_t) * n_graphs), "path step alloc");
+    CK(d_path_ell.reserve(sizeof(int2) * places), "path edges alloc");
+    CK(d_path_step.reserve(sizeof(float) * n_graphs), "path step alloc");
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "device query");
     const PathScratch ps = {d_path_order.as<uint16_t>(), d_path_order.as<uint16_t>() + P, d_path_ell.as<int4>(),
-                            reinterpret_cast<uint32_t*>(d_path_ell.as<int2>() + places), d_path_step.as<uint32_t>()};
+                            d_path_step.as<float>()};
     int min_n = max_n;
     for (const GraphInfo& g : h_graphs) min_n = std::min(min_n, g.n);
     CK(launch_paths(d_pts.as<float>(), d_graphs.as<GraphInfo>(), n_graphs, min_n, max_n, n_points, max_connect,
-                    d_edges.as<int2>(), d_edge_cnt.as<int32_t>(), d_edge_depth.as<float>(), pu, ps, d_S.as<float>(),
+                    d_edges.as<int2>(), d_edge_cnt.as<int32_t>(), d_edge_depth.as<float>(), ps, d_S.as<float>(),
                     sms, st), "paths from the edges");
     return LG_OK;
 }
@@ -1221,14 +1223,13 @@ lg_status Ctx::tune_fw() {
 
 lg_status Ctx::solve_paths() {
     Ctx* ctx = this;
-    PathUnit pu;
-    const bool from_edges = marched_as_set() && path_unit(pu);
+    const bool from_edges = marched_as_set() && by_edges();
     marched.valid = false;
     if (from_edges) {
         CK(d_edge_depth.reserve(sizeof(float) * std::max<int64_t>(edge_slots, 1)), "edge depth alloc");
         CK(launch_edge_depths(d_graphs.as<GraphInfo>(), n_graphs, max_edges, d_edges.as<int2>(),
                               d_edge_cnt.as<int32_t>(), d_S.as<float>(), d_edge_depth.as<float>(), st), "edge depths");
-        return solve_from_edges(pu);
+        return solve_from_edges();
     }
     if (fw_choice < 0) {
         lg_status s = tune_fw();
@@ -1338,11 +1339,10 @@ extern "C" lg_status lg_diffuse(lg_ctx* handle, float* diffuse_out) {
 }
 
 lg_status Ctx::solve_all() {
-    PathUnit pu;
-    const bool from_edges = path_unit(pu);
+    const bool from_edges = by_edges() && depths_near();
     lg_status s = from_edges ? march_to_edges() : march_edges();
     if (s != LG_OK) return s;
-    s = from_edges ? solve_from_edges(pu) : solve_paths();
+    s = from_edges ? solve_from_edges() : solve_paths();
     if (s != LG_OK) return s;
     paths_solved = true;
     s = vertex_light();
@@ -1980,12 +1980,11 @@ lg_status Ctx::frame_enqueue(double point_voxel_size, const lg_camera* camera) {
     lg_status s = render_count_early(camera);
     if (s == LG_OK) s = build_edges();
     mark(1);
-    PathUnit pu;
-    const bool from_edges = path_unit(pu);
+    const bool from_edges = by_edges() && depths_near();
     if (s == LG_OK) s = from_edges ? march_to_edges() : march_edges();
     mark(2);
     if (s == LG_OK) {
-        s = from_edges ? solve_from_edges(pu) : solve_paths();
+        s = from_edges ? solve_from_edges() : solve_paths();
         paths_solved = s == LG_OK;
     }
     mark(3);

@@ -198,19 +198,21 @@ struct Ctx {
     std::vector<int32_t> h_dart_cnt;
     lg_status march_edges();
     lg_status solve_paths();
-    // The solve from the edges (k_paths.cu), where path_unit says so, instead
+    // The solve from the edges (k_paths.cu), where by_edges says so, instead
     // of Floyd-Warshall; march_to_edges is march_edges without the matrix, for
-    // the calls between whose stages nobody sees it
-    bool path_unit(PathUnit& pu) const;
+    // the calls between whose stages nobody sees it. depths_near: what an edge's
+    // march can give under the settings suits it
+    bool by_edges() const;
+    bool depths_near() const;
     // What march_edges left in the matrices: depths cut off for this extinction
     // and cutoff, until a solve or another set of graphs takes their place
     struct Marched {
-        bool valid = false;
+        bool valid = false, near = false;
         double by[4] = {0.0, 0.0, 0.0, 0.0};
     } marched;
     bool marched_as_set() const;
     lg_status march_to_edges();
-    lg_status solve_from_edges(const PathUnit& pu);
+    lg_status solve_from_edges();
     lg_status vertex_light();
     lg_status diffuse();
     lg_status solve_all();

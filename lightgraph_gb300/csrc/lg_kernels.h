@@ -57,28 +57,19 @@ cudaError_t launch_vertex_light(const DevScene& sc, const float* pts, const Grap
                                 int n_graphs, int max_n, float* L, cudaStream_t st);
 
 // All-pairs paths of the graphs from their edges' depths W into the matrices S
-// (distances, diagonal 0, padding inf). Scratch: perm and rank a half-word per
-// point, ell path_stride / 2 places and rest path_stride words a point, step a
-// word per graph.
-// Distances are counted in units: `far` of them and more are no path, and an
-// edge no longer than `longest` added to far still fits 32 bits.
-struct PathUnit {
-    double per_unit;  // units in a depth of 1: per / 2^64 * 2^exponent
-    uint64_t per;
-    int exponent;
-    float longest;
-    uint32_t far;
-};
+// (distances, diagonal 0, padding inf). No depth is negative, and those that are
+// not 0 lie within a factor of kPathDepthRange. Scratch: perm and rank a
+// half-word per point, ell path_stride / 2 places a point, step a word per graph.
 struct PathScratch {
     uint16_t *perm, *rank;
     int4* ell;
-    uint32_t* rest;
-    uint32_t* step;
+    float* step;
 };
-constexpr int kPathMaxPoints = 9200;  // K = 4 distances of a graph in shared memory
+constexpr double kPathDepthRange = 1048576.0;
+constexpr int kPathMaxPoints = 8928;  // K = 4 distances of a graph in shared memory
 int path_stride(int max_connect);
 cudaError_t launch_paths(const float* pts, const GraphInfo* graphs, int n_graphs, int min_n, int max_n, int64_t n_points,
-                         int max_connect, const int2* edges, const int32_t* edge_cnt, const float* W, const PathUnit& pu,
+                         int max_connect, const int2* edges, const int32_t* edge_cnt, const float* W,
                          const PathScratch& ps, float* S, int sms, cudaStream_t st);
 
 // The edges' depths W from the matrices S.

@@ -93,3 +93,104 @@ def test_matrix_of_other_settings(gpu_ctx, scene):
     gpu_ctx.set_fw_schedule(-1)
     for a, b in zip(out[-1], out[4]):
         assert np.array_equal(a, b)
+
+
+def rewired(sc, factor=1.0, span=0.0, **shader):
+    """The scene with its extinction times factor, without dropout, its density
+    falling by e^-span across the volume."""
+    import copy
+    out = copy.copy(sc)
+    out.shader, out.opts = copy.deepcopy(sc.shader), copy.deepcopy(sc.opts)
+    out.shader.setScattering(tuple(factor * s for s in sc.shader.scattering))
+    out.shader.setAbsorption(tuple(factor * a for a in sc.shader.absorption))
+    for k, v in shader.items():
+        setattr(out.shader, k, v)
+    out.opts.cutoff = 0.0
+    if span:
+        out.density = copy.copy(sc.density)
+        fall = np.exp(-span * np.linspace(0.0, 1.0, sc.density.values.shape[2]))
+        out.density.values = np.ascontiguousarray(sc.density.values * fall, np.float32)
+    return out
+
+
+def paths(ctx, sc, clouds, radius, schedule):
+    scenes.load_into(ctx, sc)
+    ctx.set_fw_schedule(schedule)
+    ctx.build_graphs(clouds, [np.float32(radius) ** 2] * len(clouds), 12)
+    S = ctx.march_edges(want=True)
+    out = S, ctx.solve_paths(want=True), ctx.fw_schedule()[0]
+    ctx.set_fw_schedule(-1)
+    return out
+
+
+@pytest.mark.parametrize("kw", [
+    dict(), dict(factor=1e-2), dict(factor=1e-4), dict(factor=1e-6),     # thin volumes
+    dict(factor=1000.0),                                                # no transmittance along most paths
+    dict(span=9.0, scatter_density_min=3e-5, density_max=1.0),          # densities and so depths far apart
+    dict(scatter_density_min=3e-5, density_max=1.0, density_scale=0.01),  # many edges at the least density
+])
+@pytest.mark.parametrize("n, radius", [(503, 0.2), (2051, 0.11)])
+def test_distances(gpu_ctx, scene, kw, n, radius):
+    """The distances against FP64: as the FP32 oracle's within 1e-6 and finite
+    where those are, off by no more than Floyd-Warshall's in the mean, and at
+    most by five halves of an FP32 unit (one rounding of 2^-24, and as many as
+    the longest sums differ by where two paths nearly tie)."""
+    sc = rewired(scene, **kw)
+    clouds = [cloud(scene, n, 11)]
+    S, dist, used = paths(gpu_ctx, sc, clouds, radius, -1)
+    assert used == -1  # from the edges
+    S4, fw, _ = paths(gpu_ctx, sc, clouds, radius, 4)
+    assert np.array_equal(S[0], S4[0])
+    true = po.apsp_dijkstra_f64(S[0])
+    np.fill_diagonal(true, 0.0)
+    fin = np.isfinite(true)
+    if n < 1000:
+        ref = po.fw_minplus_f32(S[0])
+        np.fill_diagonal(ref, 0.0)
+        assert np.array_equal(np.isfinite(ref), fin)
+        assert np.allclose(dist[0][fin], ref[fin], rtol=1e-6, atol=0)
+    assert np.array_equal(np.isfinite(dist[0]), fin) and np.array_equal(dist[0], dist[0].T)
+    on = fin & (true > 1e-30)
+    assert np.all(dist[0][fin & ~on] == 0.0)
+    off = np.abs(dist[0][on] / true[on] - 1.0)
+    off_fw = np.abs(fw[0][on] / true[on] - 1.0)
+    print("PATHS", n, kw, "rms %.2e / %.2e max %.2e / %.2e" % (np.sqrt(np.mean(off ** 2)), np.sqrt(np.mean(off_fw ** 2)), off.max(), off_fw.max()))
+    assert np.mean(off ** 2) <= np.mean(off_fw ** 2)
+    assert off.max() <= 2.5 * 2.0 ** -23
+    if kw.get("factor") == 1000.0:
+        assert true[on].max() * min(-e for e in sc.shader.getExtinction()) > 400.0
+
+
+def test_depths_too_far_apart(gpu_ctx, scene):
+    """Depths that may lie further apart than 2^20: Floyd-Warshall, the same
+    bits as with a schedule pinned, also where they were marched so and the
+    settings have changed since."""
+    for least in (0.0, 1e-6):
+        sc = rewired(scene, span=9.0, scatter_density_min=least, density_max=10.0)
+        clouds = [cloud(scene, 307, 12)]
+        _, dist, used = paths(gpu_ctx, sc, clouds, 0.2, -1)
+        assert used >= 0
+        _, fw, _ = paths(gpu_ctx, sc, clouds, 0.2, 4)
+        assert np.array_equal(dist[0], fw[0])
+        scenes.load_into(gpu_ctx, sc)
+        gpu_ctx.build_graphs(clouds, [np.float32(0.2) ** 2], 12)
+        gpu_ctx.march_edges()
+        later = rewired(scene, span=9.0)
+        gpu_ctx.set_shader(later.shader)
+        assert np.array_equal(gpu_ctx.solve_paths(want=True)[0], fw[0])
+
+
+def test_diffusion_under_another_extinction(gpu_ctx, scene):
+    """Radiances diffused again under a smaller extinction than that of the
+    solve: as with a schedule pinned."""
+    thick = rewired(scene, factor=1000.0)
+    out = []
+    for schedule in (-1, 4):
+        scenes.load_into(gpu_ctx, thick)
+        gpu_ctx.set_fw_schedule(schedule)
+        gpu_ctx.build_graphs([cloud(scene, 400, 12)], [np.float32(0.2) ** 2], 12)
+        gpu_ctx.solve_graphs()
+        gpu_ctx.set_shader(rewired(scene, factor=0.1).shader)
+        out.append(gpu_ctx.diffuse(want=True))
+    gpu_ctx.set_fw_schedule(-1)
+    assert np.allclose(out[0], out[1], rtol=1e-4, atol=1e-7) and out[1].max() > 0
