@@ -1788,11 +1788,14 @@ lg_status Ctx::render(const lg_camera* c) {
         if ((int64_t)total * n_lights > INT32_MAX)
             return fail(LG_ERR_INVALID, "more than 2^31 shadow-ray groups in one frame");
         CK(d_tasks.reserve(sizeof(ShadowTask) * std::max<int64_t>(total, 1)), "shadow task alloc");
+        frame_tasks = total;
     }
     const int64_t cap = std::min<int64_t>((int64_t)(d_tasks.bytes / sizeof(ShadowTask)), INT32_MAX / n_lights);
     RayOrder ro{};
     ro.rb = ray_bins(sc);
-    env_order(sc, cap, ro.env);
+    // (by the tasks of this frame, or of the run a capture follows: cap is what
+    // the largest frame so far needed)
+    env_order(sc, frame_tasks, ro.env);
     ro.n_keys = 0;
     for (int k = 0; k < ro.rb.n; ++k) ro.n_keys += ro.rb.b[k].nkeys;
     if (ro.n_keys >= INT32_MAX) return fail(LG_ERR_INVALID, "more than 2^31 shadow-ray order keys");

@@ -94,6 +94,7 @@ struct Ctx {
     std::vector<GraphInfo> h_graphs;
     std::vector<float> h_pts;
     double point_voxel_size_cache = -1.0;
+    int64_t frame_tasks = 0;  // shading samples of the last frame that was not captured
     bool graphs_built = false, paths_solved = false, light_done = false, diffuse_done = false;
     DevBuf d_pts, d_graphs, d_pt_graph, d_cand, d_cand_cnt, d_pairs, d_edges, d_edge_cnt, d_adj, d_adj_off;
     DevBuf d_S, d_L, d_D, d_part, d_colw, d_fw;

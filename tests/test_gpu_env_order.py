@@ -50,3 +50,60 @@ def test_sorted_rays_match_oracle(gpu_ctx, dtype, samples):
     ref = o.render((lo, dims, vals), rows=rows)
     for i, name in enumerate(("rgba", "direct", "scatter", "emission")):
         assert rel_rmse(getattr(films, name)[rows], ref[i][rows]) <= 1e-3, name
+
+
+def test_small_frames_after_a_large_one(gpu_ctx):
+    """Whether a frame's rays are sorted is decided by that frame: after a large
+    one a thumbnail over the same volume takes the launches and gives the bits
+    that it does on a context of its own, captured or not."""
+    from lightgraph_gb300 import Context
+    n, depth, h = 520, 72, 0.0025
+    v = np.full((depth, n, n), 0.3, np.float32)
+    grid = Grid(v, (-264, -264, -40), h)
+    sh = Shader()
+    sh.setScattering((0.05, 0.05, 0.05))
+    sh.setAbsorption(0.005)
+    lights = [Light.parse("dir:0:1,0.9,0.8:1.0:-35,25,0"), Light.parse("env:20:1,1,1:0.5:2:sky")]
+    sky = scenes.envmap(64, 32)
+    pts = [scenes.points(np.full((64, 64, 64), 0.5, np.float32), 0.002, 64, 5)]
+    r2 = [np.float32(0.05) ** 2]
+
+    def settings(w, hgt):
+        return SceneSettings(width=w, height=hgt, samples=1, camTranslate=(0.0, 0.0, 1.4), iter=1, seed=3)
+
+    def load(ctx):
+        ctx.upload_density(grid)
+        ctx.upload_temperature(None)
+        ctx.set_shader(sh)
+        ctx.set_settings(settings(48, 32))
+        ctx.set_lights(lights, sky)
+        ctx.build_graphs(pts, r2, 12)
+        ctx.solve_graphs()
+        ctx.splat()
+
+    def thumbnail(ctx):
+        before = ctx.kernel_launches()
+        films = ctx.render(settings(48, 32))
+        launches = ctx.kernel_launches() - before
+        ctx.set_graph_mode(True)
+        ctx.frame_device(settings(48, 32))
+        captured = int(ctx.lib.lg_frame_launches(ctx.h))
+        ctx.frame_device(settings(48, 32))
+        replayed = ctx.films(settings(48, 32))
+        ctx.set_graph_mode(False)
+        return films, replayed, launches, captured
+
+    other = Context(0)
+    load(other)
+    films, replayed, launches, captured = thumbnail(other)
+    other.close()
+    load(gpu_ctx)
+    before = gpu_ctx.kernel_launches()
+    gpu_ctx.render(settings(640, 480))
+    assert gpu_ctx.shading_tasks() >= 4 << 20
+    assert gpu_ctx.kernel_launches() - before > launches  # sorted
+    got = thumbnail(gpu_ctx)
+    assert got[2:] == (launches, captured)
+    for name in ("rgba", "direct", "scatter", "emission"):
+        assert np.array_equal(getattr(got[0], name), getattr(films, name)), name
+        assert np.array_equal(getattr(got[1], name), getattr(replayed, name)), name
