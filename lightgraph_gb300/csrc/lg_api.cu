@@ -428,8 +428,11 @@ lg_status Ctx::upload_grid(int which, const lg_grid_desc* desc, const float* val
     int bbox[12];
     CK(cudaMemcpyAsync(bbox, small.p, sizeof bbox, cudaMemcpyDeviceToHost, st), "bbox download");
     CK(cudaStreamSynchronize(st), "grid upload sync");
-    // (the staging buffer stays: an animation uploads a grid of the same size
-    // every frame, and freeing 28 MB and allocating them again took 0.14 ms)
+    // (a staging buffer of up to kStagingKept stays: an animation uploads a grid of
+    // the same size every frame, and freeing 28 MB and allocating them again took
+    // 0.14 ms; a larger one, of which the upload itself takes 1 ms and more, is not
+    // worth its memory)
+    if (staging.bytes > kStagingKept) staging.release();
     g.has_leaves = bbox[0] <= bbox[3];
     for (int a = 0; a < 3; ++a) {
         g.bbmin[a] = g.has_leaves ? (float)(bbox[a] * 8) : 0.f;

@@ -75,6 +75,7 @@ struct Ctx {
     const GridStore& D() const { return dens_ext ? *dens_ext : dens; }
     const GridStore& T() const { return temp_ext_set ? *temp_ext : temp; }
     DevBuf staging, mask_staging, small;
+    static constexpr size_t kStagingKept = 64 << 20;  // a 256^3 grid
 
     // scene
     lg_shader shader{};

@@ -62,3 +62,20 @@ def test_boxes(gpu_ctx, dims, dtype, masked, factor):
     assert clo == rlo and cdims == rdims
     assert np.array_equal(vals != 0, rvals != 0)
     assert np.allclose(vals, rvals, rtol=1e-4, atol=1e-7)
+
+
+def test_staging_is_given_back():
+    """After an upload a context holds the records, the bitmaps and at most 64 MB
+    of staging, whatever the size of the grid."""
+    import torch
+    from lightgraph_gb300 import Context
+    ctx = Context(0)
+    ctx.upload_density(Grid(np.ones((8, 8, 8), np.float32), (0, 0, 0), 0.1), 1)  # first-use allocations
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    n = 416  # 288 MB of staging
+    ctx.upload_density(Grid(np.ones((n, n, n), np.float32), (0, 0, 0), 0.1), 1)
+    held = free - torch.cuda.mem_get_info()[0]
+    records = (n // 8 + 2) ** 3 * 512 * 16
+    ctx.close()
+    assert held <= records + (96 << 20)
