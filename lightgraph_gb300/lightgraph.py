@@ -225,7 +225,9 @@ class Grid:
 
 @dataclass
 class Films:
-    """The four Film objects of render() (src/main.cc:90-93), each H x W x 4."""
+    """The four Film objects of render() (src/main.cc:90-93), each H x W x 4.
+    Large ones are views of memory that the context uses again once the last
+    array on it is gone (_ResultBlocks); one to be resized in place is copied first."""
     rgba: np.ndarray
     direct: np.ndarray
     scatter: np.ndarray
@@ -274,6 +276,11 @@ class _ResultBlocks:
                 self.blocks.pop(0)
             return out
 
+    def clear(self) -> None:
+        """Gives the memory back: what is in use lives as long as its arrays."""
+        with self.lock:
+            self.blocks.clear()
+
 
 class Context:
     """One CUDA device and stream with the resident grids and stage buffers."""
@@ -293,6 +300,7 @@ class Context:
         if self.h:
             self.lib.lg_destroy(self.h)
             self.h = None
+            self._results.clear()
 
     def __del__(self):
         try:

@@ -6,7 +6,7 @@ import threading
 import numpy as np
 import pytest
 
-from lightgraph_gb300.lightgraph import _ResultBlocks
+from lightgraph_gb300.lightgraph import Context, _ResultBlocks
 
 
 def address(a):
@@ -69,3 +69,18 @@ def test_threads():
     for t in threads:
         t.join()
     assert not bad and len(pool.blocks) <= pool.KEEP
+
+
+def test_closed_context_keeps_none():
+    class Lib:
+        lg_destroy = staticmethod(lambda handle: None)
+
+    ctx = Context.__new__(Context)
+    ctx.lib, ctx.h, ctx._results = Lib, 1, _ResultBlocks()
+    kept, dropped = ctx._results.empty((256, 256)), ctx._results.empty((300, 300))
+    kept[...] = 4.0
+    del dropped
+    ctx.close()
+    assert not ctx._results.blocks
+    assert (kept == 4.0).all()
+    ctx.close()
