@@ -16,7 +16,8 @@
  *    serialised by an internal mutex; use one context per host thread for
  *    concurrency (the serving entry points overlap requests internally).
  *  - All work is deterministic: the same inputs give bit-identical outputs,
- *    independent of how many other requests share the GPU.
+ *    independent of how many other requests share the GPU. (Graphs solved
+ *    together are one input: see lg_set_fw_schedule.)
  *  - World/index convention (OpenVDB linear transform, uniform voxels):
  *      world = index * voxel_size + world_origin
  *    Voxel centres sit at integer index coordinates. Leaves are the aligned
@@ -376,8 +377,11 @@ uint64_t lg_frame_launches(const lg_ctx* ctx);
  * builds) with 1 or 2 CTAs per SM; 5: schedule 4 with the update tiles'
  * operands staged into shared memory by TMA bulk copies (cp.async.bulk on an
  * mbarrier) instead of through registers. Schedules 0 to 5 give the same
- * distances bit for bit. A schedule set here stays in force for later graph
- * builds until -1 is set again. */
+ * distances bit for bit, whatever graphs are loaded together. With -1 the choice
+ * is by the loaded graphs as a whole: a graph's radiances may differ in their last
+ * bits from those of the same graph in another batch. Programs that deal graphs
+ * over calls or GPUs and compare bits set a schedule, as the serving calls do. A
+ * schedule set here stays in force for later graph builds until -1 is set again. */
 lg_status lg_set_fw_schedule(lg_ctx* ctx, int schedule);
 /* The schedule in use (-1: none chosen, as while graphs are solved from their
  * edges) and the autotuner's timings (ms) of schedules 0..5 (0 for a schedule

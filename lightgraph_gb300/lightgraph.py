@@ -469,7 +469,8 @@ class Context:
         self._ck(self.lib.lg_frame_device(self.h, max_connect, point_voxel_size, C.byref(cam)))
 
     def set_fw_schedule(self, schedule: int) -> None:
-        """-1 from the edges or autotuned, 0 per-graph launches, 1/2 persistent (CTAs per SM),
+        """-1 from the edges or autotuned, by the graphs loaded together (the others
+        give a graph the same bits in any batch), 0 per-graph launches, 1/2 persistent (CTAs per SM),
         3/4 symmetric persistent (CTAs per SM), 5 = 4 with the update tiles'
         operands staged by TMA bulk copies."""
         self._ck(self.lib.lg_set_fw_schedule(self.h, schedule))

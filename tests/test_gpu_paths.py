@@ -194,3 +194,27 @@ def test_diffusion_under_another_extinction(gpu_ctx, scene):
         out.append(gpu_ctx.diffuse(want=True))
     gpu_ctx.set_fw_schedule(-1)
     assert np.allclose(out[0], out[1], rtol=1e-4, atol=1e-7) and out[1].max() > 0
+
+
+def test_graphs_dealt_over_calls(gpu_ctx, scene):
+    """Nine graphs in one call and dealt over two: the same radiances bit for bit
+    with a schedule set, and to FP32 roundings (one call goes by Floyd-Warshall,
+    the others from the edges) without."""
+    sizes = [300, 120, 257, 64, 400, 90, 333, 210, 150]
+    clouds = [cloud(scene, n, 20 + n) for n in sizes]
+    r2 = [np.float32(1.3 * n ** (-1.0 / 3.0)) ** 2 for n in sizes]
+    scenes.load_into(gpu_ctx, scene)
+    for schedule in (4, 2, -1):
+        gpu_ctx.set_fw_schedule(schedule)
+        out = []
+        for parts in ([slice(0, 9)], [slice(0, 1), slice(1, 9)]):
+            D = []
+            for part in parts:
+                gpu_ctx.build_graphs(clouds[part], r2[part], 12)
+                D.append(gpu_ctx.solve_graphs(want=True))
+            out.append(np.concatenate(D))
+        if schedule >= 0:
+            assert np.array_equal(out[0], out[1]), schedule
+        else:
+            assert np.allclose(out[0], out[1], rtol=4e-6, atol=0)
+    gpu_ctx.set_fw_schedule(-1)
