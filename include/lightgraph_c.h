@@ -420,6 +420,12 @@ lg_status lg_fw_queue_check(int n_graphs, const int32_t* sizes, int sym, int64_t
  * lg_diffuse, lg_render_frame, ...) return LG_ERR_TIMEOUT the same way when
  * a persistent solve of theirs raised its error word. */
 lg_status lg_wait_timeout_check(lg_ctx* ctx, uint32_t polls);
+/* The same for the waits between the CTAs of a cluster that throws darts (no
+ * counterpart in the reference): iteration 0 of lg_scatter_points, each wait
+ * ending after `polls` looks (1 to 2^24). Returns LG_ERR_TIMEOUT, as
+ * lg_scatter_points does, when one gave up (the context stays usable), LG_OK if
+ * none had to. */
+lg_status lg_dart_wait_check(lg_ctx* ctx, const lg_scatter_opts* opts, uint32_t polls);
 
 /* ------------------------------------------------------------------------- */
 /* Image files without the OpenEXR library                                   */

@@ -615,7 +615,6 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_dart(DevGrid g, D
 
 constexpr int kDartChunk = 16 * kMtN / 3;  // candidates a chunk
 constexpr int kDartSlots = 3;              // chunks between the helpers and the first CTA
-constexpr uint32_t kDartPolls = 1u << 22;  // of a shared-memory word, some 40 cycles each
 
 // First CTA. A slot holds the offsets of the candidates that passed and a bit
 // for each; ready: the number of the chunk in it, plus one.
@@ -664,11 +663,11 @@ __device__ __forceinline__ uint32_t acquire(const uint32_t* p) {
     return v;
 }
 // The warp waits until *p has reached v, or until *stop is set; false then or
-// after kDartPolls looks.
-__device__ __forceinline__ bool wait_for(const uint32_t* p, uint32_t v, const uint32_t* stop) {
+// after `polls` looks.
+__device__ __forceinline__ bool wait_for(const uint32_t* p, uint32_t v, const uint32_t* stop, uint32_t polls) {
     int ok = 0;
     if ((threadIdx.x & 31) == 0)
-        for (uint32_t k = 0; k < kDartPolls && !(stop && acquire(stop)); ++k)
+        for (uint32_t k = 0; k < polls && !(stop && acquire(stop)); ++k)
             if (acquire(p) >= v) {
                 ok = 1;
                 break;
@@ -705,7 +704,7 @@ __device__ __forceinline__ void dart_helper(const DevGrid& g, const DartParams& 
         if (twister >= 0 && c + n < chunks)
             for (int k = 0; k < n; ++k) mt_next_chunk<16>(sh.words[(buf + k) % 3], sh.words[(buf + k + 1) % 3], twister);
         const int slot = c % kDartSlots;
-        const bool free = c < kDartSlots || wait_for(&sh.used, c + 1 - kDartSlots, &sh.stop);
+        const bool free = c < kDartSlots || wait_for(&sh.used, c + 1 - kDartSlots, &sh.stop, prm.polls);
         while (free) {
             int j = 0;
             if (lane == 0) j = atomicAdd(&sh.claim[par], 64);
@@ -765,7 +764,7 @@ __global__ void __launch_bounds__(1024, 1) k_dart_cluster(DevGrid g, DartParams 
     // warps w of nw: those left go to the queue; false if the chunk did not come
     auto hint_tests = [&](uint32_t c, int j0, int j1, float hint_m2, int queue, int w, int nw) {
         const int slot = c % kDartSlots;
-        if (!wait_for(&sh.ready[slot], c + 1, nullptr)) return false;
+        if (!wait_for(&sh.ready[slot], c + 1, nullptr, prm.polls)) return false;
         for (int k = (j0 >> 5) + w; 32 * k < j1; k += nw) {
             const int j = 32 * k + lane;
             const bool in = ((sh.bits[slot][k] >> lane) & 1u) && j >= j0 && j < j1;

@@ -742,7 +742,7 @@ extern "C" lg_status lg_randgen_draws(uint32_t seed, int64_t n, float* out, uint
     return LG_OK;
 }
 
-lg_status Ctx::scatter_points(const lg_scatter_opts& o, int first_iter, int n_iter) {
+lg_status Ctx::scatter_points(const lg_scatter_opts& o, int first_iter, int n_iter, uint32_t polls) {
     Ctx* ctx = this;
     const GridStore& gs = D();
     if (!gs.valid) return fail(LG_ERR_STATE, "no density grid uploaded");
@@ -778,6 +778,7 @@ lg_status Ctx::scatter_points(const lg_scatter_opts& o, int first_iter, int n_it
     prm.target = o.target_size;
     prm.batch = batch;
     prm.hard_limit = o.hard_limit;
+    prm.polls = polls;
     prm.cutoff = o.density_cutoff;
     prm.min_dist_sq0 = min_dist * min_dist;
     prm.seed_base = o.seed_base;
@@ -2107,6 +2108,14 @@ extern "C" lg_status lg_wait_timeout_check(lg_ctx* handle, uint32_t polls) {
     CK(cudaStreamSynchronize(ctx->st), "sync");
     if (w[2] == 1u && w[1] != 0u) return ctx->fail(LG_ERR_TIMEOUT, "the bounded wait gave up after %u polls", polls);
     return ctx->fail(LG_ERR_STATE, "the bounded wait did not give up (error word %u, outcome %u)", w[1], w[2]);
+}
+
+extern "C" lg_status lg_dart_wait_check(lg_ctx* handle, const lg_scatter_opts* opts, uint32_t polls) {
+    Ctx* ctx = reinterpret_cast<Ctx*>(handle);
+    GUARD(ctx);
+    if (!opts) return ctx->fail(LG_ERR_INVALID, "null scatter options");
+    if (polls < 1 || polls > (1u << 24)) return ctx->fail(LG_ERR_INVALID, "polls must be in [1, 2^24]");
+    return ctx->scatter_points(*opts, 0, 1, polls);
 }
 
 extern "C" lg_status lg_fw_queue_check(int n_graphs, const int32_t* sizes, int sym, int64_t* n_items) {

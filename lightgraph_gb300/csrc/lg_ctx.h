@@ -194,7 +194,7 @@ struct Ctx {
                           int max_connect);
     lg_status build_edges();
     // LightGraph::scatterPoints for n_iter iterations into h_dart_* (host)
-    lg_status scatter_points(const lg_scatter_opts& o, int first_iter, int n_iter);
+    lg_status scatter_points(const lg_scatter_opts& o, int first_iter, int n_iter, uint32_t polls = kDartPolls);
     DevBuf d_dart_pts, d_dart_cnt, d_dart_m2, d_dart_expected;
     std::vector<float> h_dart_pts, h_dart_m2;
     std::vector<int32_t> h_dart_cnt;

@@ -293,7 +293,9 @@ struct DartParams {
     // of the point and hint grids, rounding slack of a radius
     float bb_hi[3], bb_lo[3], bb_err[3], wo_hi[3], wo_lo[3], inv_h_lo;
     float cell_inv[3], hint_inv[3], cell_slack;
+    uint32_t polls;  // looks at a shared-memory word, some 40 cycles each, before a cluster's wait gives up
 };
+constexpr uint32_t kDartPolls = 1u << 22;
 // expected: the expected sizes at the scatter_count / batch radius updates;
 // out_pts: n_iter x hard_limit x 3 floats; out_last_m2: the squared minimum
 // distance of each iteration's last accepted point.

@@ -5,7 +5,7 @@ points, bit for bit, in the same order) and so must the connect radii."""
 import numpy as np
 import pytest
 
-from lightgraph_gb300 import lightgraph as lgm, scenes
+from lightgraph_gb300 import _capi, lightgraph as lgm, scenes
 from oracle import pyoracle as po
 
 pytestmark = pytest.mark.gpu
@@ -133,3 +133,21 @@ def test_early_ends_on_clusters(gpu_ctx, target):
             assert np.array_equal(np.asarray(q), np.asarray(r2)[:n], equal_nan=True)
             for i in range(n):
                 assert np.array_equal(pts[i].view(np.uint32), alone[i].view(np.uint32)), (n, i)
+
+
+def test_waits_between_ctas_give_up(gpu_ctx):
+    """A cluster whose first CTA does not wait for the first chunk's words (one
+    look at them) ends with an error and leaves the context usable; with the
+    limit in use no wait runs out."""
+    import ctypes
+    sc = scenes.small(n_points=16, res=64)
+    scenes.load_into(gpu_ctx, sc)
+    opts = lgm.scatter_opts(scatter_count=60000)
+    check = lambda polls: gpu_ctx.lib.lg_dart_wait_check(gpu_ctx.h, ctypes.byref(opts), polls)  # noqa: E731
+    for _ in range(3):
+        assert check(1) == _capi.LG_ERR_TIMEOUT
+        assert b"ran out" in gpu_ctx.lib.lg_last_error(gpu_ctx.h)
+        check_iterations(gpu_ctx, sc, opts, 0, 2)
+    assert check(1 << 22) == _capi.LG_OK
+    assert check(0) == _capi.LG_ERR_INVALID
+    assert check((1 << 24) + 1) == _capi.LG_ERR_INVALID
