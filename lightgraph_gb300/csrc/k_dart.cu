@@ -12,8 +12,8 @@
 //
 // Here one CTA, or a cluster, runs one iteration and reproduces that sequence
 // exactly. A CTA takes the candidates a chunk at a time (3328 or 1664 of them),
-// radius update falls inside one, so that the radius is one number in each
-// range:
+// in ranges: a range is a chunk, or a part of one where a radius update falls
+// inside it, so that the radius is one number in each range:
 //   1. warps take groups of 64 candidates from a counter: position in FP32 index
 //      space, one cell record, density test. A candidate whose density or
 //      cell the FP32 error leaves undecided is tested again with an index

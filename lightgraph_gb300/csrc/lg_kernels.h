@@ -183,16 +183,15 @@ struct ShadowTask {
 };
 static_assert(sizeof(ShadowTask) == 32, "ShadowTask is two 16-byte words");
 size_t pixel_sample_bytes();
-// Ordering of the shadow rays of one light: tasks are counting-sorted by a
+// Ordering of the shadow rays of a distant or point light: tasks are counting-sorted by a
 // key that groups rays which cross the same part of the volume, so the rays
 // in flight share cache lines and the lanes of a warp walk similar paths.
 //   kind 0 (distant light, parallel rays): (u, v) bin of the start point
 //          projected on the plane normal to the ray direction D, in Morton
 //          order, then the depth bin along D;
 //   kind 1 (point light, rays through O): cube-map face and (s, t) bin of the
-//          direction from O to the start point, then the distance bin;
-//   kind 2 (environment light, random directions): task order in buckets of
-//          2^shift tasks.
+//          direction from O to the start point, then the distance bin.
+// (EnvOrder: environment lights.)
 struct RayBin {
     int kind, ns, nd;         // ns: (u, v) or (s, t) bins per side (power of two), nd: depth bins
     int light;                // the scene's light
@@ -201,7 +200,7 @@ struct RayBin {
     float u0, v0, inv_bs;     // kind 0: projected origin, 1 / bin size
     float d0, inv_ds;         // depth origin, 1 / depth bin size
     int64_t key_off, nkeys;   // this light's keys in the combined histogram
-    // Occupancy bound per light-space bin (kinds 0 and 1; null: none). A
+    // Occupancy bound per light-space bin (null: none). A
     // distant light's shadow ray stays in its (u, v) column and a point
     // light's in its cube-map cone, so no leaf lies on the ray past the
     // column's largest leaf depth - d0 (kind 0, ns x ns, v major) or closer to
@@ -237,9 +236,6 @@ inline int64_t bound_entries(const RayBin& b) {
 cudaError_t launch_render_count(const DevScene& sc, const DevCamera& cam, const DevScatterGrid& sg, int32_t* counts,
                                 unsigned long long* claim, int sms, cudaStream_t st,
                                 bool short_ctas = false);
-// Shadow-ray ordering buffers: key_counts and key_offsets hold rb's keys,
-// key_scan the scan's block sums (keys / 1024 + 2), order n_lights * units
-// (units of kRayUnit tasks).
 // Order of an environment light's shadow rays, a light sample at a time: by
 // direction (octahedral bins, 2^dir_bits a side), then by the start's cell
 // (2^cell_bits a side over the leaf bbox, Morton order). keys and order hold a
@@ -251,6 +247,9 @@ struct EnvOrder {
     int32_t* order;
     int64_t n_keys;  // 0: the rays stay in task order
 };
+// Shadow-ray ordering buffers: key_counts and key_offsets hold rb's keys,
+// key_scan the scan's block sums (keys / 1024 + 2), order n_lights * units
+// (units of kRayUnit tasks).
 struct RayOrder {
     RayBins rb;
     int64_t n_keys;
@@ -275,7 +274,8 @@ cudaError_t launch_render_shade(const DevScene& sc, const DevCamera& cam, const 
 cudaError_t launch_exclusive_scan(const int32_t* in, int64_t n, int32_t* out, int32_t* block_sums, int32_t* total,
                                   cudaStream_t st);
 
-// Dart throwing (LightGraph::scatterPoints), one CTA per iteration.
+// Dart throwing (LightGraph::scatterPoints), a cluster of CTAs or one CTA an
+// iteration.
 struct DartParams {
     uint32_t scatter_count, target, batch, hard_limit;
     float cutoff, min_dist_sq0;
