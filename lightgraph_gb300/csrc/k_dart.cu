@@ -696,7 +696,7 @@ __device__ __forceinline__ void dart_helper(const DevGrid& g, const DartParams& 
         for (int k = 0; k <= h; ++k) mt_next_chunk<16>(sh.words[(buf + k) % 3], sh.words[(buf + k + 1) % 3], twister);
     buf = (buf + h + 1) % 3;
     __syncthreads();
-    const uint32_t chunks = (prm.scatter_count + kDartChunk - 1) / kDartChunk;
+    const uint32_t chunks = (uint32_t)(((uint64_t)prm.scatter_count + kDartChunk - 1) / kDartChunk);
     int par = 0;
     for (uint32_t c = (uint32_t)h; c < chunks; c += n, par ^= 1) {
         const uint32_t* cur = sh.words[buf];

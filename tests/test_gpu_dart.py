@@ -151,3 +151,12 @@ def test_waits_between_ctas_give_up(gpu_ctx):
     assert check(1 << 22) == _capi.LG_OK
     assert check(0) == _capi.LG_ERR_INVALID
     assert check((1 << 24) + 1) == _capi.LG_ERR_INVALID
+
+
+def test_largest_candidate_counts(gpu_ctx):
+    """Up to 2^32 - 1 candidates an iteration, which ends at its target."""
+    sc = scenes.small(n_points=16, res=64)
+    scenes.load_into(gpu_ctx, sc)
+    for count in (2 ** 32 - 3328, 2 ** 32 - 3327, 2 ** 32 - 1):
+        opts = lgm.scatter_opts(scatter_count=count, target_size=40, hard_limit=50, min_dist_mult=0.1)
+        check_iterations(gpu_ctx, sc, opts, 0, 2)
