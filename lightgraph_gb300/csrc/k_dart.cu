@@ -40,7 +40,7 @@
 // 44.6 ms for 48 iterations of 1M candidates (256^3 cumulus); this form takes
 // 4.8 ms, and 500 iterations 16.4 ms instead of 76. Where there are SMs to
 // spare a cluster runs an iteration (k_dart_cluster): words and density tests
-// go ahead on the other CTAs, and the first one's hint tests beside the walk: 3.6 ms.
+// go ahead on the other CTAs, and the first one's hint tests beside the walk: 3.7 ms.
 #include <algorithm>
 #include <cmath>
 
@@ -910,7 +910,7 @@ cudaError_t launch_dart(const DevGrid& g, DartParams prm, int n_iter, const uint
     prm.inv_h_lo = (float)(1.0 / prm.h - (double)prm.inv_h_f);
     prm.cell_slack = extent * 1e-6f;
     // Clusters of three CTAs, or two, as long as all run at once (24 iterations:
-    // 4.6 -> 3.0 ms, 48: 4.8 -> 3.6 ms). As long as every iteration gets an SM of its own, the chain of its ranges
+    // 4.6 -> 3.0 ms, 48: 4.8 -> 3.7 ms). As long as every iteration gets an SM of its own, the chain of its ranges
     // is what takes the time: 1024 threads and chunks of 3328 candidates shorten
     // it; past that, two CTAs of 512 threads with chunks of 1664 on an SM fill
     // each other's waits.
