@@ -95,9 +95,9 @@ def test_matrix_of_other_settings(gpu_ctx, scene):
         assert np.array_equal(a, b)
 
 
-def rewired(sc, factor=1.0, span=0.0, **shader):
+def rewired(sc, factor=1.0, span=0.0, step=None, **shader):
     """The scene with its extinction times factor, without dropout, its density
-    falling by e^-span across the volume."""
+    falling by e^-span across the volume, marched in steps of `step` voxels."""
     import copy
     out = copy.copy(sc)
     out.shader, out.opts = copy.deepcopy(sc.shader), copy.deepcopy(sc.opts)
@@ -106,6 +106,8 @@ def rewired(sc, factor=1.0, span=0.0, **shader):
     for k, v in shader.items():
         setattr(out.shader, k, v)
     out.opts.cutoff = 0.0
+    if step:
+        out.opts.step = (1.0, step)
     if span:
         out.density = copy.copy(sc.density)
         fall = np.exp(-span * np.linspace(0.0, 1.0, sc.density.values.shape[2]))
@@ -126,6 +128,8 @@ def paths(ctx, sc, clouds, radius, schedule):
 @pytest.mark.parametrize("kw", [
     dict(), dict(factor=1e-2), dict(factor=1e-4), dict(factor=1e-6),     # thin volumes
     dict(factor=1000.0),                                                # no transmittance along most paths
+    dict(scattering=(0.002, 0.1, 1.0)),                                 # channels far apart
+    dict(step=4.0),                                                     # edges without a sample: depth 0
     dict(span=9.0, scatter_density_min=3e-5, density_max=1.0),          # densities and so depths far apart
     dict(scatter_density_min=3e-5, density_max=1.0, density_scale=0.01),  # many edges at the least density
 ])
@@ -151,6 +155,8 @@ def test_distances(gpu_ctx, scene, kw, n, radius):
         assert np.allclose(dist[0][fin], ref[fin], rtol=1e-6, atol=0)
     assert np.array_equal(np.isfinite(dist[0]), fin) and np.array_equal(dist[0], dist[0].T)
     on = fin & (true > 1e-30)
+    if "step" in kw:
+        assert np.sum(S[0] == 0.0) > n / 2 and np.any(on)  # both kinds of edges
     assert np.all(dist[0][fin & ~on] == 0.0)
     off = np.abs(dist[0][on] / true[on] - 1.0)
     off_fw = np.abs(fw[0][on] / true[on] - 1.0)
@@ -218,3 +224,9 @@ def test_graphs_dealt_over_calls(gpu_ctx, scene):
         else:
             assert np.allclose(out[0], out[1], rtol=4e-6, atol=0)
     gpu_ctx.set_fw_schedule(-1)
+
+
+def test_channels_far_apart(gpu_ctx, scene):
+    """Radiances under extinctions a hundred times apart, as the oracle's."""
+    solve(gpu_ctx, rewired(scene, scattering=(0.002, 0.1, 1.0), absorption=(0.001, 0.02, 0.1)),
+          [cloud(scene, 301, 14)], [0.2], 12)
